@@ -12,6 +12,127 @@ namespace {
 
 using namespace mcpg_api;
 
+// ---------------- ranked max-min products (maxmin_ranked.cu) ----------------
+#ifndef MCPG_RANKED_MIN
+#define MCPG_RANKED_MIN 256
+#endif
+// The lists and the order of one operand.
+struct RankedSet {
+    mcpg::RankedLists L{};
+    int *rank = nullptr, *perm = nullptr;
+    bool built = false;
+};
+// The scratch of one API call's ranked products.
+struct Ranked {
+    bool on = false;
+    int64_t owners = 0, cols = 0, k = 0;  // largest of the call's products
+    float *XT = nullptr, *P = nullptr;
+    mcpg::RankedPending* pending = nullptr;
+    int64_t cap = 0;
+    unsigned long long* cnt = nullptr;  // [0]: NaN seen, [1..]: a pending count per product
+    int used = 1;
+    RankedSet set[2];
+};
+constexpr int RANKED_COUNTERS = 8;
+
+// Decides whether this call's products take the ranked form, and lays out its scratch.  Dense below
+// MCPG_RANKED_MIN candidates or rows (the ranked form's six launches cost more than one small
+// product), above the list kernel's 32,768 candidates or the finishing kernel's row buffer, where
+// the scratch cannot be had, and in a stream capture that would have to allocate it.
+void ranked_begin(mcpg_handle* h, Ranked& r, int64_t owners, int64_t cols, int64_t k, int lists) {
+    r = Ranked{};
+    if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || owners < 8 || k > 32768 || owners > 50000 || cols > 50000) return;
+    const int64_t lx = round_up(std::max(owners, cols), 128);
+    const int64_t rows = std::max(owners, cols);
+    const int64_t pitch = mcpg::ranked_list_cap(k);
+    r.cap = std::max<int64_t>(4096, owners * cols / 64);
+    const size_t lbytes = (size_t)rows * (size_t)pitch * sizeof(uint2) + (size_t)rows * 5 * sizeof(int);
+    struct { int slot; size_t bytes; void* p; } need[] = {
+        {S_RK_CNT, RANKED_COUNTERS * sizeof(unsigned long long), nullptr},
+        {S_RK_XT, (size_t)k * (size_t)lx * sizeof(float), nullptr},
+        {S_RK_P, (size_t)rows * (size_t)lx * sizeof(float), nullptr},
+        {S_RK_PEND, (size_t)r.cap * sizeof(mcpg::RankedPending), nullptr},
+        {S_RK_L0, lbytes, nullptr},
+        {S_RK_L1, lists > 1 ? lbytes : 0, nullptr},
+    };
+    bool grow = false;
+    for (auto& q : need) grow |= q.bytes > h->cap[q.slot];
+    if (grow) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
+        if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return;
+        }
+    }
+    for (auto& q : need)
+        if (q.bytes && scratch(h, q.slot, q.bytes, &q.p) != MCPG_OK) return;
+    r.cnt = (unsigned long long*)need[0].p;
+    r.XT = (float*)need[1].p;
+    r.P = (float*)need[2].p;
+    r.pending = (mcpg::RankedPending*)need[3].p;
+    for (int s = 0; s < lists; ++s) {
+        RankedSet& q = r.set[s];
+        char* p = (char*)need[4 + s].p;
+        q.L.entries = (uint2*)p;
+        q.L.pitch = pitch;
+        p += (size_t)rows * (size_t)pitch * sizeof(uint2);
+        q.L.count = (int*)p;
+        q.L.bound = (float*)(q.L.count + rows);
+        q.L.strength = (int*)(q.L.bound + rows);
+        q.rank = q.L.strength + rows;
+        q.perm = q.rank + rows;
+    }
+    if (cudaMemsetAsync(r.cnt, 0, RANKED_COUNTERS * sizeof(unsigned long long), h->stream) != cudaSuccess) return;
+    r.owners = owners; r.cols = cols; r.k = k;
+    r.on = true;
+}
+
+// One product p (C and/or R of MM_PLAIN / MM_RATIO) with p.A as the owner operand and its lists in
+// set s; swap: p.B owns (its rows carry the lists), which suits an A whose rows have no
+// pronounced largest values.  Falls back to the exhaustive kernel on the device.
+int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p, int mode, bool symm, bool swap) {
+    if (!r.on || r.used >= RANKED_COUNTERS) {
+        PROF(h, "maxmin");
+        CK(h, mcpg::launch_maxmin(p, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
+        return MCPG_OK;
+    }
+    PROF(h, "maxmin");
+    RankedSet& q = r.set[s];
+    mcpg::RankedArgs a{};
+    a.O = swap ? p.B : p.A; a.ldo = swap ? p.ldb : p.lda;
+    a.X = swap ? p.A : p.B; a.ldx = swap ? p.lda : p.ldb;
+    a.owners = (int)(swap ? p.cols : p.rows);
+    a.cols = (int)(swap ? p.rows : p.cols);
+    a.k = (int)p.k_len;
+    if (!q.built) {
+        CK(h, mcpg::launch_ranked_lists(a.O, a.ldo, a.owners, a.k, q.L, r.cnt, h->stream, &h->launches), "lists kernel");
+        if (symm) CK(h, mcpg::launch_ranked_order(q.L, a.owners, q.rank, q.perm, h->stream, &h->launches), "order kernel");
+        q.built = true;
+    }
+    a.L = q.L;
+    a.ldt = round_up(a.cols, 128);
+    CK(h, mcpg::launch_ranked_transpose(a.X, a.ldx, a.cols, a.k, symm ? q.perm : nullptr, r.XT, a.ldt, r.cnt, h->stream,
+                                        &h->launches),
+       "transpose kernel");
+    a.XT = r.XT;
+    a.perm = symm ? q.perm : nullptr;
+    a.P = r.P;
+    a.ldp = round_up(swap ? a.owners : a.cols, 128);
+    a.direct = symm || !swap;
+    a.mirror = symm || swap;
+    a.pending = r.pending; a.pending_cap = r.cap;
+    a.pending_n = r.cnt + r.used++;
+    a.nan = r.cnt;
+    CK(h, mcpg::launch_ranked_walk(a, symm ? 1 : 0, h->stream, &h->launches), "ranked max-min kernel");
+    mcpg::MaxminParams d = p;
+    d.run_above = a.pending_n; d.run_cap = (unsigned long long)a.pending_cap; d.run_nan = a.nan;
+    CK(h, mcpg::launch_maxmin(d, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
+    CK(h, mcpg::launch_ranked_finish(a, symm ? q.rank : nullptr, symm ? q.rank : nullptr, p.rows, p.cols, p.C, p.ldc,
+                                     p.E, p.lde, mode == mcpg::MM_RATIO ? p.R : nullptr, p.ldr, h->stream, &h->launches),
+       "ranked finish kernel");
+    return MCPG_OK;
+}
+
 int maxmin_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb, int64_t rows, int64_t cols,
                int64_t k, float* C, int64_t ldc) {
     if (rows < 0 || cols < 0 || k < 0) return fail(h, MCPG_ERR_ARG, "maxmin: negative size");
@@ -34,11 +155,9 @@ int maxmin_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int6
     p.A = a; p.lda = la; p.B = b; p.ldb = lb;
     p.rows = rows; p.cols = cols; p.k_len = k;
     p.C = C; p.ldc = ldc;
-    {
-        PROF(h, "maxmin");
-        CK(h, mcpg::launch_maxmin(p, mcpg::MM_PLAIN, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
-    }
-    return MCPG_OK;
+    Ranked r;
+    ranked_begin(h, r, rows, cols, k, 1);
+    return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, symm, false);
 }
 
 int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len, int symmetrize, float* Mout,
@@ -54,37 +173,26 @@ int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len
     int rc = aligned_view(h, A, lda, n, n, S_IN0, &a, &la);
     if (rc) return rc;
     const int64_t ldt = round_up(n, 32);
+    Ranked rk;
+    ranked_begin(h, rk, n, n, n, path_len == 4 ? 2 : 1);
     mcpg::MaxminParams p{};
     p.rows = n; p.cols = n; p.k_len = n;
     if (path_len == 2) {
         p.A = a; p.lda = la; p.B = a; p.ldb = la;
         p.C = Mout; p.ldc = ldm; p.E = a; p.lde = la; p.R = Rout; p.ldr = ldr;
-        if (Rout) {
-            {
-                PROF(h, "maxmin");
-                CK(h, mcpg::launch_maxmin(p, mcpg::MM_RATIO, 1, h->stream, &h->launches), "maxmin+ratio kernel");
-            }
-        } else {
-            {
-                PROF(h, "maxmin");
-                CK(h, mcpg::launch_maxmin(p, mcpg::MM_PLAIN, 1, h->stream, &h->launches), "maxmin kernel");
-            }
-        }
-        return MCPG_OK;
+        return ranked_product(h, rk, 0, p, Rout ? mcpg::MM_RATIO : mcpg::MM_PLAIN, true, false);
     }
     // M1 = A (x) A (symmetric)
     void* m1;
     rc = scratch(h, S_M1, (size_t)(n * ldt) * sizeof(float), &m1);
     if (rc) return rc;
     p.A = a; p.lda = la; p.B = a; p.ldb = la; p.C = (float*)m1; p.ldc = ldt;
-    {
-        PROF(h, "maxmin");
-        CK(h, mcpg::launch_maxmin(p, mcpg::MM_PLAIN, 1, h->stream, &h->launches), "maxmin kernel (M1)");
-    }
+    if ((rc = ranked_product(h, rk, 0, p, mcpg::MM_PLAIN, true, false))) return rc;
     const float* X1 = (const float*)m1;
     mcpg::MaxminParams q{};
     q.rows = n; q.cols = n; q.k_len = n;
     int sym2;
+    const int set2 = path_len == 4 ? 1 : 0;  // whose lists: M1's, or A's again
     if (path_len == 3) {  // A (x) M1, InnerProduct(A, M1), not assumed symmetric
         q.A = a; q.lda = la; q.B = X1; q.ldb = ldt; sym2 = 0;
     } else {              // M1 (x) M1, symmetric
@@ -95,10 +203,7 @@ int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len
         rc = scratch(h, S_M2, (size_t)(n * ldt) * sizeof(float), &m2);
         if (rc) return rc;
         q.C = (float*)m2; q.ldc = ldt;
-        {
-            PROF(h, "maxmin");
-            CK(h, mcpg::launch_maxmin(q, mcpg::MM_PLAIN, sym2, h->stream, &h->launches), "maxmin kernel (M2)");
-        }
+        if ((rc = ranked_product(h, rk, set2, q, mcpg::MM_PLAIN, sym2 != 0, false))) return rc;
         float* sym = Mout;
         int64_t lds = ldm;
         if (!sym) {  // reuse M1's slot: M1 is no longer needed
@@ -117,18 +222,7 @@ int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len
         return MCPG_OK;
     }
     q.C = Mout; q.ldc = ldm; q.E = a; q.lde = la; q.R = Rout; q.ldr = ldr;
-    if (Rout) {
-        {
-            PROF(h, "maxmin");
-            CK(h, mcpg::launch_maxmin(q, mcpg::MM_RATIO, sym2, h->stream, &h->launches), "maxmin+ratio kernel");
-        }
-    } else {
-        {
-            PROF(h, "maxmin");
-            CK(h, mcpg::launch_maxmin(q, mcpg::MM_PLAIN, sym2, h->stream, &h->launches), "maxmin kernel");
-        }
-    }
-    return MCPG_OK;
+    return ranked_product(h, rk, set2, q, Rout ? mcpg::MM_RATIO : mcpg::MM_PLAIN, sym2 != 0, false);
 }
 
 // Intermediates of the first phase of the two-phase DPI (a multiple of the max-min
@@ -633,29 +727,23 @@ int maxmins_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float* M
         if ((rc = scratch(h, S_M1, (size_t)(n * l1) * sizeof(float), &p))) return rc;
         m1 = (float*)p;
     }
+    Ranked rk;
+    ranked_begin(h, rk, n, n, n, M3 || R4 ? 2 : 1);
     mcpg::MaxminParams p{};
     p.rows = n; p.cols = n; p.k_len = n;
     p.A = a; p.lda = la; p.B = a; p.ldb = la; p.C = m1; p.ldc = l1; p.E = a; p.lde = la; p.R = R2; p.ldr = ldr2;
-    {
-        PROF(h, "maxmin");
-        CK(h, mcpg::launch_maxmin(p, R2 ? mcpg::MM_RATIO : mcpg::MM_PLAIN, 1, h->stream, &h->launches),
-           "maxmin kernel (M1)");
-    }
+    if ((rc = ranked_product(h, rk, 0, p, R2 ? mcpg::MM_RATIO : mcpg::MM_PLAIN, true, false))) return rc;
     if (M2 || R3) {
         mcpg::MaxminParams q{};
         q.rows = n; q.cols = n; q.k_len = n;
         q.A = a; q.lda = la; q.B = m1; q.ldb = l1; q.C = M2; q.ldc = ld2; q.E = a; q.lde = la; q.R = R3; q.ldr = ldr3;
-        PROF(h, "maxmin");
-        CK(h, mcpg::launch_maxmin(q, R3 ? mcpg::MM_RATIO : mcpg::MM_PLAIN, 0, h->stream, &h->launches),
-           "maxmin kernel (M2)");
+        if ((rc = ranked_product(h, rk, 0, q, R3 ? mcpg::MM_RATIO : mcpg::MM_PLAIN, false, false))) return rc;
     }
     if (M3 || R4) {
         mcpg::MaxminParams q{};
         q.rows = n; q.cols = n; q.k_len = n;
         q.A = m1; q.lda = l1; q.B = m1; q.ldb = l1; q.C = M3; q.ldc = ld3; q.E = a; q.lde = la; q.R = R4; q.ldr = ldr4;
-        PROF(h, "maxmin");
-        CK(h, mcpg::launch_maxmin(q, R4 ? mcpg::MM_RATIO : mcpg::MM_PLAIN, 1, h->stream, &h->launches),
-           "maxmin kernel (M3)");
+        if ((rc = ranked_product(h, rk, 1, q, R4 ? mcpg::MM_RATIO : mcpg::MM_PLAIN, true, false))) return rc;
     }
     if (M1 && m1 != M1) CK(h, mcpg::launch_copy2d(m1, l1, M1, ld1, n, n, h->stream), "copy2d");
     return MCPG_OK;

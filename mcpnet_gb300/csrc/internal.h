@@ -57,11 +57,56 @@ struct MaxminParams {
     // MM_DPI / MM_DPI1 on a permuted input P A P^T: output (i, j) goes to
     // C / mask [perm[i]][perm[j]] (device, nullable = identity)
     const int* perm;
+    // run only when *run_above (device) exceeds run_cap or *run_nan is set (nullable: always run)
+    const unsigned long long* run_above; unsigned long long run_cap;
+    const unsigned long long* run_nan;
 };
 
 // symmetric != 0: A == B (same rows), rows == cols; only tiles on or above the
 // diagonal are computed and mirrored (C is symmetric for any A in that case).
 cudaError_t launch_maxmin(const MaxminParams& p, int mode, int symmetric, cudaStream_t stream, int64_t* launches);
+
+// ---- max-min products with ordered candidates (maxmin_ranked.cu) ----
+// Per owner row: its largest entries as (value, k) in descending order, padded to a multiple
+// of 8 with -inf; bound >= every entry not listed; strength orders the rows.
+struct RankedLists {
+    uint2* entries; int64_t pitch;  // rows x pitch
+    int* count;
+    float* bound;
+    int* strength;
+};
+struct RankedPending {
+    int32_t o, p;
+    float m;
+};
+struct RankedArgs {
+    const float* O; int64_t ldo;  // owner operand, owners x k, 16-byte aligned rows
+    const float* X; int64_t ldx;  // other operand, cols x k, 16-byte aligned rows
+    const float* XT; int64_t ldt; // its transpose in column order perm, ldt a multiple of 128
+    int owners, cols, k;
+    RankedLists L;                // of O, in natural row order
+    const int* perm;              // column p is row perm[p] of X (nullable: p)
+    float* P; int64_t ldp;        // direct: P[o][p], mirror: P[p][o]
+    int direct, mirror;
+    RankedPending* pending; int64_t pending_cap;
+    unsigned long long* pending_n;  // appended outputs; above pending_cap: the ranked form gave up
+    const unsigned long long* nan;  // nonzero: an operand holds a NaN, and it gave up too
+};
+int ranked_list_cap(int64_t k);
+cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64_t k, const RankedLists& L,
+                                unsigned long long* nan, cudaStream_t st, int64_t* launches);
+cudaError_t launch_ranked_order(const RankedLists& L, int64_t n, int* rank, int* perm, cudaStream_t st,
+                                int64_t* launches);
+cudaError_t launch_ranked_transpose(const float* X, int64_t ldx, int64_t rows, int64_t k, const int* perm, float* XT,
+                                    int64_t ldt, unsigned long long* nan, cudaStream_t st, int64_t* launches);
+// symmetric: O == X, owners in the order of perm, only columns at or after the owner.
+cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t st, int64_t* launches);
+// C[i][j] = P[rrank ? rrank[i] : i][crank ? crank[j] : j] and R = ratio(E, C), each nullable;
+// nothing when the ranked form gave up.
+cudaError_t launch_ranked_finish(const RankedArgs& a, const int* rrank, const int* crank, int64_t rows, int64_t cols,
+                                 float* C, int64_t ldc, const float* E, int64_t lde, float* R, int64_t ldr,
+                                 cudaStream_t st, int64_t* launches);
+
 cudaError_t launch_ratio(const float* A, int64_t lda, const float* M, int64_t ldm, int64_t rows, int64_t cols,
                          float* R, int64_t ldr, cudaStream_t stream, int64_t* launches);
 // Second phase of the two-phase DPI: for every pending pair, continue the max-min over

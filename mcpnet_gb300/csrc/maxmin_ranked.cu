@@ -1,0 +1,486 @@
+// Max-min products with the candidates k visited in descending order of one operand.
+//
+//   C[i][j] = max_k min(O[i][k], X[j][k])
+//
+// For an output (i, j) only the k with O[i][k] > C[i][j] matter, and on similarity
+// matrices they are few: with independent rows the maximum sits near the
+// sqrt(k)-th largest value of each row.  So each owner row i gets the list of its
+// largest entries, (value, k) in descending order, and a warp walks that list for 128
+// columns j at once: acc = max(acc, min(value, X[j][k])).  When every lane's acc has
+// reached the next value of the list, no later k can raise it: the outputs are final.
+// A selection has no rounding, so the bits are those of the exhaustive product.
+//
+// The walk reads X transposed, XT[k][j], 512 contiguous bytes per (k, warp): it is bound
+// by L2-to-SM bandwidth (4 bytes per candidate), and visits a few percent of the
+// n^3 candidates.  Column blocks are the slow grid axis, so the k x 128 slab that the
+// resident CTAs read stays in L2.
+//
+// A symmetric product (O == X) needs each pair once, and the pair is cheaper from the
+// row whose large values are smaller (the capacity is limited by that row: few of its
+// entries exceed it, while a strongly connected row has many).  Rows are ordered by
+// the strength of their 2 sqrt(k)-th largest value, weakest first, and the walk runs on
+// the upper triangle of the product in that order, in a scratch matrix P that the last
+// kernel reads back in gene order (with the MCP ratio fused).
+//
+// Outputs whose list ends too early go to a pending list and are completed one warp each
+// from the other row's list, and where that is not enough from both whole rows.  If
+// more outputs stay open than the pending list holds (data without such structure: many
+// ties, closures), or an operand holds a NaN, a device-side count tells the exhaustive kernel
+// (maxmin.cu), which is always enqueued behind and otherwise returns at once, to run.  No
+// host synchronisation: the sequence can be captured and stays asynchronous.
+//
+// Measured on MI-like matrices (symmetric product with ratio, whole call; exhaustive form ->
+// this one): 20,000 genes 338 -> 19.7 ms (walk 13.5, lists 2.9, finish 1.9, transpose 1.1 ms);
+// M1..M3 with ratios at 2,000 genes 1.79 -> 0.48 ms; 300 genes, one product, 71 -> 66 us.
+#include <float.h>
+#include <math.h>
+
+#include "common.cuh"
+#include "internal.h"
+
+namespace mcpg {
+namespace {
+
+constexpr unsigned FULL = 0xffffffffu;
+constexpr int LIST_TPB = 512;
+constexpr int LIST_MAX = 1024;   // longest list (sort buffer)
+constexpr int BATCH = 8;         // list entries between two exit tests
+constexpr int COLS = 128;        // columns of a warp: a float4 per lane
+constexpr int OWN = 8;           // owners (warps) of a CTA
+
+// Order-preserving map of the float bits to signed integers (-0 below +0).
+__device__ __forceinline__ int okey(float f) {
+    const int u = __float_as_int(f);
+    return u ^ ((u >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float okey_value(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
+// Whether the ranked form gave up: too many pending outputs, or a NaN operand (the exhaustive
+// kernel behind it runs on the same condition).
+__device__ __forceinline__ bool gave_up(const RankedArgs& a) {
+    return *(const volatile unsigned long long*)a.pending_n > (unsigned long long)a.pending_cap || *a.nan != 0;
+}
+// 16 bytes through the read-only path; volatile keeps a batch's loads together and in front
+// of their uses.
+__device__ __forceinline__ float4 ldg4(const float* p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+// One CTA per owner row: the row's keys sit in registers (EPT per thread); a bisection on the
+// key counts entries above a pivot until between want and cap are, they are compacted
+// and sorted (bitonic, key then index).  bound[i] = an upper bound of every entry not
+// listed (-inf when all are).  Entries are padded to a multiple of BATCH with -inf.
+template <int EPT>
+__global__ void __launch_bounds__(LIST_TPB) lists_kernel(const float* __restrict__ O, int64_t ldo, int rows, int k,
+                                                         int want, int cap, int strength_at, RankedLists L,
+                                                         unsigned long long* any_nan) {
+    __shared__ unsigned long long buf[LIST_MAX];
+    __shared__ int wcount[LIST_TPB / 32];
+    __shared__ int fill;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i = blockIdx.x;
+    const float* row = O + (int64_t)i * ldo;
+    int key[EPT];
+    bool nan = false;
+    int mn = INT_MAX, mx = INT_MIN;
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) {
+        const int c = tid + e * LIST_TPB;
+        key[e] = INT_MIN;  // below okey(-inf): never counted
+        if (c < k) {
+            const float v = row[c];
+            nan |= (v != v);
+            key[e] = okey(v);
+            mn = min(mn, key[e]);
+            mx = max(mx, key[e]);
+        }
+    }
+    if (nan) *any_nan = 1;  // NaN has no place in the order: the exhaustive kernel takes the product
+    auto block_sum = [&](int v) {
+        v = __reduce_add_sync(FULL, v);
+        __syncthreads();
+        if (lane == 0) wcount[warp] = v;
+        __syncthreads();
+        int s = lane < LIST_TPB / 32 ? wcount[lane] : 0;
+        return __reduce_add_sync(FULL, s);
+    };
+    auto above = [&](int pivot) {
+        int c = 0;
+#pragma unroll
+        for (int e = 0; e < EPT; ++e) c += key[e] > pivot;
+        return block_sum(c);
+    };
+    {
+        mn = __reduce_min_sync(FULL, mn);
+        mx = __reduce_max_sync(FULL, mx);
+        __shared__ int smn[LIST_TPB / 32], smx[LIST_TPB / 32];
+        if (lane == 0) { smn[warp] = mn; smx[warp] = mx; }
+        __syncthreads();
+        mn = __reduce_min_sync(FULL, lane < LIST_TPB / 32 ? smn[lane] : INT_MAX);
+        mx = __reduce_max_sync(FULL, lane < LIST_TPB / 32 ? smx[lane] : INT_MIN);
+    }
+    // invariant: above(lo) > cap, above(hi) < want
+    int pivot, n_above;
+    if (k <= cap) {
+        pivot = INT_MIN;  // everything is listed
+        n_above = k;
+    } else {
+        long long lo = (long long)mn - 1, hi = mx;
+        pivot = mx;
+        n_above = 0;
+        while (hi - lo > 1) {
+            const int mid = (int)(lo + (hi - lo) / 2);
+            const int c = above(mid);
+            if (c > cap) lo = mid;
+            else {
+                hi = mid;
+                pivot = mid;
+                n_above = c;
+                if (c >= want) break;
+            }
+        }
+    }
+    // entries above the pivot, then entries equal to it as far as the list has room
+    if (tid == 0) fill = 0;
+    __syncthreads();
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 1 && (k <= cap || n_above >= want)) break;
+#pragma unroll
+        for (int e = 0; e < EPT; ++e) {
+            const bool take = key[e] != INT_MIN && (pass == 0 ? key[e] > pivot : key[e] == pivot);
+            const unsigned b = __ballot_sync(FULL, take);
+            if (!b) continue;
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&fill, __popc(b));
+            base = __shfl_sync(FULL, base, 0);
+            const int at = base + __popc(b & ((1u << lane) - 1u));
+            if (take && at < cap)
+                buf[at] = ((unsigned long long)((unsigned)key[e] ^ 0x80000000u) << 32) | (unsigned)(tid + e * LIST_TPB);
+        }
+        __syncthreads();
+    }
+    const int count = min(fill, cap);
+    int p2 = 32;
+    while (p2 < count) p2 <<= 1;
+    for (int t = count + tid; t < p2; t += LIST_TPB) buf[t] = 0;
+    __syncthreads();
+    for (int s = 2; s <= p2; s <<= 1)
+        for (int j = s >> 1; j > 0; j >>= 1) {
+            for (int t = tid; t < p2 / 2; t += LIST_TPB) {
+                const int x = ((t & ~(j - 1)) << 1) | (t & (j - 1)), y = x | j;
+                const unsigned long long a = buf[x], b = buf[y];
+                if ((a < b) == ((x & s) == 0)) {
+                    buf[x] = b;
+                    buf[y] = a;
+                }
+            }
+            __syncthreads();
+        }
+    const int padded = (count + BATCH - 1) / BATCH * BATCH;
+    uint2* out = L.entries + (int64_t)i * L.pitch;
+    for (int t = tid; t < padded; t += LIST_TPB) {
+        uint2 e = make_uint2(0xff800000u, 0u);  // -inf
+        if (t < count) {
+            const unsigned long long v = buf[t];
+            e.x = __float_as_uint(okey_value((int)((unsigned)(v >> 32) ^ 0x80000000u)));
+            e.y = (unsigned)v;
+        }
+        out[t] = e;
+    }
+    if (tid == 0) {
+        const bool all = count == k;
+        L.count[i] = count;
+        L.bound[i] = all ? -INFINITY : okey_value(pivot);
+        L.strength[i] = strength_at < count ? (int)((unsigned)(buf[strength_at] >> 32) ^ 0x80000000u)
+                                            : (all ? INT_MIN : pivot);
+    }
+}
+
+// rank[i] = position of row i by ascending strength (ties by index), perm = its inverse.
+__global__ void __launch_bounds__(256) order_kernel(const int* __restrict__ strength, int n, int* __restrict__ rank,
+                                                    int* __restrict__ perm) {
+    const int i = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const int s = strength[i];
+    int c = 0;
+    for (int j = lane; j < n; j += 32) {
+        const int t = strength[j];
+        c += (t < s) || (t == s && j < i);
+    }
+    c = __reduce_add_sync(FULL, c);
+    if (lane == 0) {
+        rank[i] = c;
+        perm[c] = i;
+    }
+}
+
+// XT[k][p] = X[perm ? perm[p] : p][k]; columns p in [rows, ldt) are +inf (they never keep a
+// warp from its exit).
+__global__ void __launch_bounds__(256) transpose_kernel(const float* __restrict__ X, int64_t ldx, int rows, int k,
+                                                        const int* __restrict__ perm, float* __restrict__ XT,
+                                                        int64_t ldt, unsigned long long* any_nan) {
+    __shared__ float tile[32][33];
+    const int p0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+    for (int r = ty; r < 32; r += 8) {
+        const int p = p0 + r, c = k0 + tx;
+        float v = INFINITY;
+        if (p < rows && c < k) v = X[(int64_t)(perm ? perm[p] : p) * ldx + c];
+        if (v != v) *any_nan = 1;
+        tile[r][tx] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = ty; r < 32; r += 8)
+        if (k0 + r < k) XT[(int64_t)(k0 + r) * ldt + p0 + tx] = tile[tx][r];
+}
+
+// One warp per (owner, 128 columns).  SYM: owners and columns in strength order, columns
+// at or after the owner only.
+template <bool SYM>
+__global__ void __launch_bounds__(OWN * 32) walk_kernel(const RankedArgs a) {
+    __shared__ float tile[OWN][COLS + 4];
+    if (__syncthreads_or(threadIdx.x == 0 && gave_up(a))) return;
+    const int o0 = blockIdx.x * OWN, p0 = blockIdx.y * COLS;
+    if (SYM && p0 + COLS <= o0) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int o = o0 + w, p = p0 + lane * 4;
+    if (o < a.owners && !(SYM && p0 + COLS <= o)) {
+        const int i = SYM ? a.perm[o] : o;
+        const uint4* list = reinterpret_cast<const uint4*>(a.L.entries + (int64_t)i * a.L.pitch);
+        const int count = a.L.count[i];
+        const float bound = a.L.bound[i];
+        const float* col = a.XT + p;
+        // columns before the owner belong to other warps
+        const bool live0 = !SYM || p >= o, live1 = !SYM || p + 1 >= o, live2 = !SYM || p + 2 >= o,
+                   live3 = !SYM || p + 3 >= o;
+        float4 acc = make_float4(live0 ? -INFINITY : INFINITY, live1 ? -INFINITY : INFINITY,
+                                 live2 ? -INFINITY : INFINITY, live3 ? -INFINITY : INFINITY);
+        bool open = count == 0;
+        for (int t = 0; t < count; t += BATCH) {
+            uint4 e[BATCH / 2];
+            float4 b[BATCH];
+#pragma unroll
+            for (int u = 0; u < BATCH / 2; ++u) e[u] = __ldg(list + t / 2 + u);
+#pragma unroll
+            for (int u = 0; u < BATCH / 2; ++u) {
+                b[2 * u] = ldg4(col + (int64_t)e[u].y * a.ldt);
+                b[2 * u + 1] = ldg4(col + (int64_t)e[u].w * a.ldt);
+            }
+            // the largest entry not yet visited
+            const float next = t + BATCH < count ? __uint_as_float(__ldg(&list[t / 2 + BATCH / 2].x)) : bound;
+#pragma unroll
+            for (int u = 0; u < BATCH / 2; ++u) {
+                const float v0 = __uint_as_float(e[u].x), v1 = __uint_as_float(e[u].z);
+                acc.x = fmax3(acc.x, fmin2(v0, b[2 * u].x), fmin2(v1, b[2 * u + 1].x));
+                acc.y = fmax3(acc.y, fmin2(v0, b[2 * u].y), fmin2(v1, b[2 * u + 1].y));
+                acc.z = fmax3(acc.z, fmin2(v0, b[2 * u].z), fmin2(v1, b[2 * u + 1].z));
+                acc.w = fmax3(acc.w, fmin2(v0, b[2 * u].w), fmin2(v1, b[2 * u + 1].w));
+            }
+            const int kn = okey(next);
+            open = okey(acc.x) < kn || okey(acc.y) < kn || okey(acc.z) < kn || okey(acc.w) < kn;
+            if (!__any_sync(FULL, open)) break;
+        }
+        if (__any_sync(FULL, open)) {
+            const int kn = okey(bound);
+            const bool u0 = p < a.cols && okey(acc.x) < kn, u1 = p + 1 < a.cols && okey(acc.y) < kn;
+            const bool u2 = p + 2 < a.cols && okey(acc.z) < kn, u3 = p + 3 < a.cols && okey(acc.w) < kn;
+            const unsigned below = (1u << lane) - 1u;
+            const unsigned m0 = __ballot_sync(FULL, u0), m1 = __ballot_sync(FULL, u1), m2 = __ballot_sync(FULL, u2),
+                           m3 = __ballot_sync(FULL, u3);
+            unsigned long long base = 0;
+            const int total = __popc(m0) + __popc(m1) + __popc(m2) + __popc(m3);
+            if (lane == 0 && total) base = atomicAdd(a.pending_n, (unsigned long long)total);
+            base = __shfl_sync(FULL, base, 0);
+            auto put = [&](bool u, unsigned long long at, int pp, float m) {
+                if (u && at < (unsigned long long)a.pending_cap) a.pending[at] = RankedPending{o, pp, m};
+            };
+            put(u0, base + __popc(m0 & below), p, acc.x);
+            base += __popc(m0);
+            put(u1, base + __popc(m1 & below), p + 1, acc.y);
+            base += __popc(m1);
+            put(u2, base + __popc(m2 & below), p + 2, acc.z);
+            base += __popc(m2);
+            put(u3, base + __popc(m3 & below), p + 3, acc.w);
+        }
+        if (a.direct) {
+            float* dst = a.P + (int64_t)o * a.ldp + p;
+            if (live0) *reinterpret_cast<float4*>(dst) = acc;  // ldp covers the last column block
+            else {
+                if (live1) dst[1] = acc.y;
+                if (live2) dst[2] = acc.z;
+                if (live3) dst[3] = acc.w;
+            }
+        }
+        if (a.mirror) *reinterpret_cast<float4*>(&tile[w][lane * 4]) = acc;
+    }
+    if (a.mirror) {
+        __syncthreads();
+        // P[p][o0 .. o0 + 7]: two float4 per row p
+        const int r = threadIdx.x >> 1, h = (threadIdx.x & 1) * 4;
+        const int pp = p0 + r;
+        if (pp < a.cols) {
+            float* dst = a.P + (int64_t)pp * a.ldp + o0 + h;
+            const int last = o0 + h + 3;
+            if (last < a.owners && (!SYM || pp >= last)) {
+                *reinterpret_cast<float4*>(dst) = make_float4(tile[h][r], tile[h + 1][r], tile[h + 2][r], tile[h + 3][r]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (o0 + h + q < a.owners && (!SYM || pp >= o0 + h + q)) dst[q] = tile[h + q][r];
+            }
+        }
+    }
+}
+
+// One warp per pending output: the other row's list (SYM), then both whole rows.
+template <bool SYM>
+__global__ void __launch_bounds__(256) pending_kernel(const RankedArgs a) {
+    if (gave_up(a)) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t count = (int64_t)*a.pending_n;
+    for (int64_t x = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < count; x += nw) {
+        const RankedPending d = a.pending[x];
+        const int i = SYM ? a.perm[d.o] : d.o, j = a.perm ? a.perm[d.p] : d.p;
+        const float* ro = a.O + (int64_t)i * a.ldo;
+        const float* rx = a.X + (int64_t)j * a.ldx;
+        float acc = d.m;
+        float bound = a.L.bound[i];
+        bool open = true;
+        if (SYM) {
+            const uint2* list = a.L.entries + (int64_t)j * a.L.pitch;
+            const int c = a.L.count[j];
+            const float bj = a.L.bound[j];
+            for (int t = 0; t < c && open; t += 32) {
+                if (t + lane < c) {
+                    const uint2 e = __ldg(list + t + lane);
+                    acc = fmax2(acc, fmin2(__uint_as_float(e.x), __ldg(ro + e.y)));
+                }
+                const float next = t + 32 < c ? __uint_as_float(__ldg(&list[t + 32].x)) : bj;
+                open = !__any_sync(FULL, okey(acc) >= okey(next));
+            }
+            bound = fminf(bound, bj);
+            if (open) open = !__any_sync(FULL, okey(acc) >= okey(bound));
+        }
+        const int kb = okey(bound);
+        for (int t = 0; t < a.k && open; t += 128) {
+            const int c = t + lane * 4;
+            if (c + 3 < a.k) {
+                const float4 u = __ldg(reinterpret_cast<const float4*>(ro + c));
+                const float4 v = __ldg(reinterpret_cast<const float4*>(rx + c));
+                acc = fmax3(acc, fmin2(u.x, v.x), fmin2(u.y, v.y));
+                acc = fmax3(acc, fmin2(u.z, v.z), fmin2(u.w, v.w));
+            } else {
+                for (int q = c; q < a.k; ++q) acc = fmax2(acc, fmin2(ro[q], rx[q]));
+            }
+            open = !__any_sync(FULL, okey(acc) >= kb);
+        }
+        const int best = __reduce_max_sync(FULL, okey(acc));
+        if (lane == 0) {
+            const float v = okey_value(best);
+            if (a.direct) a.P[(int64_t)d.o * a.ldp + d.p] = v;
+            if (a.mirror) a.P[(int64_t)d.p * a.ldp + d.o] = v;
+        }
+    }
+}
+
+__device__ __forceinline__ float ratio_value(float a, float m) {  // ratio_kernel, combine.hpp:210-222
+    return (fabsf(a) < FLT_EPSILON) ? 0.0f : (fabsf(m) < FLT_EPSILON) ? FLT_MAX : __fdiv_rn(a, m);
+}
+
+// C[i][j] = P[rrank ? rrank[i] : i][crank ? crank[j] : j], R = ratio(E, C).
+template <bool GATHER>
+__global__ void __launch_bounds__(512) finish_kernel(const RankedArgs a, const int* __restrict__ rrank,
+                                                     const int* __restrict__ crank, int rows, int cols,
+                                                     float* __restrict__ C, int64_t ldc, const float* __restrict__ E,
+                                                     int64_t lde, float* __restrict__ R, int64_t ldr) {
+    extern __shared__ float prow[];
+    if (__syncthreads_or(threadIdx.x == 0 && gave_up(a))) return;
+    for (int i = blockIdx.x; i < rows; i += gridDim.x) {
+        const float* src = a.P + (int64_t)(rrank ? rrank[i] : i) * a.ldp;
+        if (GATHER) {
+            __syncthreads();
+            for (int j = threadIdx.x * 4; j < cols; j += 512 * 4)  // ldp is a multiple of 128
+                *reinterpret_cast<float4*>(prow + j) = *reinterpret_cast<const float4*>(src + j);
+            __syncthreads();
+        }
+        for (int j = threadIdx.x; j < cols; j += 512) {
+            const float v = GATHER ? prow[crank[j]] : src[j];
+            if (C) C[i * ldc + j] = v;
+            if (R) R[i * ldr + j] = ratio_value(E[i * lde + j], v);
+        }
+    }
+}
+
+int isqrt_ceil(int64_t v) { return (int)ceil(sqrt((double)v)); }
+
+}  // namespace
+
+int ranked_list_cap(int64_t k) {
+    // four square roots of the candidate count cover 99 % of the outputs of the measured matrices
+    int64_t c = (4 * (int64_t)isqrt_ceil(k) + 31) / 32 * 32;
+    return (int)(c > LIST_MAX ? LIST_MAX : c);
+}
+
+cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64_t k, const RankedLists& L,
+                                unsigned long long* nan, cudaStream_t st, int64_t* launches) {
+    const int cap = ranked_list_cap(k), want = cap * 3 / 4, at = 2 * isqrt_ceil(k);
+    if (k > (int64_t)LIST_TPB * 64 || L.pitch < cap) return cudaErrorInvalidValue;
+    if (launches) ++*launches;
+    const unsigned g = (unsigned)rows;
+    if (k <= LIST_TPB * 4) lists_kernel<4><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, L, nan);
+    else if (k <= LIST_TPB * 16) lists_kernel<16><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, L, nan);
+    else if (k <= LIST_TPB * 40) lists_kernel<40><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, L, nan);
+    else lists_kernel<64><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, L, nan);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ranked_order(const RankedLists& L, int64_t n, int* rank, int* perm, cudaStream_t st,
+                                int64_t* launches) {
+    if (launches) ++*launches;
+    order_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, st>>>(L.strength, (int)n, rank, perm);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ranked_transpose(const float* X, int64_t ldx, int64_t rows, int64_t k, const int* perm, float* XT,
+                                    int64_t ldt, unsigned long long* nan, cudaStream_t st, int64_t* launches) {
+    if (launches) ++*launches;
+    dim3 grid((unsigned)(ldt / 32), (unsigned)ceil_div(k, 32));
+    transpose_kernel<<<grid, 256, 0, st>>>(X, ldx, (int)rows, (int)k, perm, XT, ldt, nan);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t st, int64_t* launches) {
+    if (launches) *launches += 2;
+    dim3 grid((unsigned)ceil_div(a.owners, OWN), (unsigned)ceil_div(a.cols, COLS));
+    if (symmetric) walk_kernel<true><<<grid, OWN * 32, 0, st>>>(a);
+    else walk_kernel<false><<<grid, OWN * 32, 0, st>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const unsigned g = 152 * 8;
+    if (symmetric) pending_kernel<true><<<g, 256, 0, st>>>(a);
+    else pending_kernel<false><<<g, 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ranked_finish(const RankedArgs& a, const int* rrank, const int* crank, int64_t rows, int64_t cols,
+                                 float* C, int64_t ldc, const float* E, int64_t lde, float* R, int64_t ldr,
+                                 cudaStream_t st, int64_t* launches) {
+    if (launches) ++*launches;
+    const unsigned g = (unsigned)(rows < 152 * 16 ? rows : 152 * 16);
+    if (crank) {
+        const size_t smem = (size_t)((cols + 3) / 4 * 4) * sizeof(float);
+        cudaError_t e = cudaFuncSetAttribute(finish_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        finish_kernel<true><<<g, 512, smem, st>>>(a, rrank, crank, (int)rows, (int)cols, C, ldc, E, lde, R, ldr);
+    } else {
+        finish_kernel<false><<<g, 512, 0, st>>>(a, rrank, crank, (int)rows, (int)cols, C, ldc, E, lde, R, ldr);
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace mcpg
