@@ -13,7 +13,10 @@ struct MiPlan {
     int precision = 0, fmt = 0, split = 0, bins = 0;  // split: mcpg::TcMode
     int64_t n = 0, m = 0;
     const void* w0 = nullptr;  // FP32 sample-major or 16-bit hi weights
-    const void* w1 = nullptr;  // 16-bit lo weights, or the interleaved E4M3 H8|L8 plane (split 2)
+    const void* w1 = nullptr;  // 16-bit lo weights, or the interleaved E4M3 H8|L8 plane (split 2); FP32 with 10
+                               // bins / order 3: the (weights, first row) entries
+    int64_t ldg = 0;           // their leading dimension (genes)
+    int* irregular = nullptr;  // set where a sample has weights outside three neighbouring bins
     int64_t ld = 0;            // weight leading dimension
     double* H = nullptr;
     float* MI = nullptr;
@@ -43,16 +46,29 @@ int mi_prepare(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx
     if (precision == MCPG_MI_FP32) {
         if (bins < 2 || bins > 12)
             return fail(h, MCPG_ERR_UNSUPPORTED, "bspline_mi FP32: bins must be 2..12 (got %d)", bins);
-        const int64_t ldwt = round_up(n, 16) * bins;
-        const int64_t m_pad = round_up(m, 16);
-        void* p;
+        // three weight rows per sample (mi_rows_kernel), unless its entries do not fit the device
+        bool rows = bins == 10 && order == 3;
+        void *p, *ent = nullptr, *flag = nullptr;
+        if (rows && scratch(h, S_W1, (size_t)(mcpg::mi_rows_samples(m) * mcpg::mi_rows_genes(n)) * sizeof(float4), &ent))
+            rows = false;
+        const int64_t genes = rows ? mcpg::mi_rows_genes(n) : round_up(n, 16);
+        const int64_t ldwt = genes * bins;
+        const int64_t m_pad = rows ? mcpg::mi_rows_samples(m) : round_up(m, 16);
         if ((rc = scratch(h, S_W0, (size_t)(m_pad * ldwt) * sizeof(float), &p))) return rc;
+        if (rows && (rc = scratch(h, S_SMALL, 64, &flag))) return rc;
         CK(h, cudaMemsetAsync(p, 0, (size_t)(m_pad * ldwt) * sizeof(float), h->stream), "memset weights");
-        PROF(h, "bspline_weights");
-        CK(h, mcpg::launch_bspline_weights_fp32(X, n, m, ldx, bins, order, (float*)p, ldwt, pl.H, h->stream,
-                                                 &h->launches),
-           "bspline weights kernel");
-        pl.w0 = p;
+        if (rows) CK(h, cudaMemsetAsync(flag, 0, sizeof(int), h->stream), "memset flag");
+        {
+            PROF(h, "bspline_weights");
+            CK(h, mcpg::launch_bspline_weights_fp32(X, n, m, ldx, bins, order, (float*)p, ldwt, pl.H, h->stream,
+                                                     &h->launches),
+               "bspline weights kernel");
+            if (rows)
+                CK(h, mcpg::launch_mi_entries((const float*)p, ldwt, genes, m, (float4*)ent, (int*)flag, h->stream,
+                                              &h->launches),
+                   "weight entries kernel");
+        }
+        pl.w0 = p; pl.w1 = rows ? ent : nullptr; pl.ldg = genes; pl.irregular = (int*)flag;
         pl.ld = ldwt;
         return MCPG_OK;
     }
@@ -94,6 +110,12 @@ int mi_prepare(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx
 int mi_launch(mcpg_handle* h, const MiPlan& pl, int64_t g0, int64_t g1) {
     if (pl.precision == MCPG_MI_FP32) {
         PROF(h, "mi_fp32");
+        if (pl.w1) {
+            CK(h, mcpg::launch_mi_rows((const float*)pl.w0, pl.ld, (const float4*)pl.w1, pl.ldg, pl.irregular, pl.H,
+                                       pl.n, pl.m, pl.MI, pl.ldmi, g0, g1, h->stream, &h->launches),
+               "MI FP32 kernel");
+            return MCPG_OK;
+        }
         CK(h, mcpg::launch_mi_fp32((const float*)pl.w0, pl.ld, pl.H, pl.n, pl.m, pl.bins, pl.MI, pl.ldmi, h->stream,
                                    &h->launches, g0, g1),
            "MI FP32 kernel");
