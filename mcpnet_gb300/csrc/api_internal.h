@@ -90,6 +90,7 @@ enum Slot {
     S_SP_ST,     // split evaluation: Stouffer scores of every coefficient row at the entries
     S_DPI_PEND,  // two-phase DPI: outputs the first phase left undecided
     S_TCWORK,    // tensor-core MI: the 2-SM form's tile counters
+    S_WK,        // MI adjoint: FP32 weights, gene-bin-major
     S_RK_XT,     // ranked max-min: the transposed operand
     S_RK_P,      // ranked max-min: the product in strength order
     S_RK_L0,     // ranked max-min: candidate lists of the first operand

@@ -163,10 +163,12 @@ int mi_dev(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx, in
     return mi_finish(h, pl);
 }
 
-// MI adjoint: dX from G = dL/dMI (FP32).  Q = Gs (log2 P + 1/ln 2) is built in
-// slabs of gene tiles that fit the slab budget, contracted with the weights on
-// the plus-times twin of the max-min kernel, then pushed through the B-spline
-// derivative and the min-max scaling per gene.
+// MI adjoint: dX from G = dL/dMI (FP32).  Q = Gs (log2 P + 1/ln 2) is built for all genes
+// against a slab of genes (all of them where that fits MCPG_Q_BYTES), contracted with the
+// gene-bin-major weights, then pushed through the B-spline derivative and the min-max scaling per gene.
+#ifndef MCPG_Q_BYTES
+#define MCPG_Q_BYTES ((size_t)8 << 30)
+#endif
 int mi_bwd_dev(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx, int bins, int order,
                const float* G, int64_t ldg, float* dX, int64_t lddx) {
     if (n < 1 || m < 1) return fail(h, MCPG_ERR_ARG, "bspline_mi_bwd: need n >= 1 and m >= 1");
@@ -176,53 +178,74 @@ int mi_bwd_dev(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx
         return fail(h, MCPG_ERR_ARG, "bspline_mi_bwd: need 1 <= order <= bins <= 12, order <= 8");
     if (bins < 2) return fail(h, MCPG_ERR_UNSUPPORTED, "bspline_mi_bwd: bins must be 2..12 (got %d)", bins);
     int rc;
-    const int64_t ldwt = round_up(n, 16) * bins;
-    const int64_t m_pad = round_up(m, 16);
-    void *wt, *hd, *gs;
+    void *wt, *wk, *ent = nullptr, *flag = nullptr, *hd, *gs;
+    // three weight rows per sample (mi_rows_kernel), unless its entries do not fit the device
+    bool rows = bins == 10 && order == 3;
+    if (rows && scratch(h, S_W1, (size_t)(mcpg::mi_rows_samples(m) * mcpg::mi_rows_genes(n)) * sizeof(float4), &ent))
+        rows = false;
+    const int64_t genes = rows ? mcpg::mi_rows_genes(n) : round_up(n, 16);
+    const int64_t ldwt = genes * bins;
+    const int64_t m_pad = rows ? mcpg::mi_rows_samples(m) : round_up(m, 16);
+    const int64_t ldk = round_up(m, 128);
     if ((rc = scratch(h, S_W0, (size_t)(m_pad * ldwt) * sizeof(float), &wt))) return rc;
+    if ((rc = scratch(h, S_WK, (size_t)(n * bins * ldk) * sizeof(float), &wk))) return rc;
+    if (rows && (rc = scratch(h, S_SMALL, 64, &flag))) return rc;
     if ((rc = scratch(h, S_H, (size_t)n * sizeof(double), &hd))) return rc;
     if ((rc = scratch(h, S_GS, (size_t)n * sizeof(float), &gs))) return rc;
+    // slabs of genes j: one for all genes (each pair's Q is then computed once), else 2 GB
+    const int64_t step = 32;
+    int64_t slab = round_up(n, step);
+    void* q = nullptr;
+    auto q_bytes = [&](int64_t g) { return (size_t)(n * bins) * (size_t)round_up(g * bins, 128) * sizeof(float); };
+    if (q_bytes(slab) > (rows ? MCPG_Q_BYTES : (size_t)2 << 30) || scratch(h, S_Q, q_bytes(slab), &q)) {
+        slab = (int64_t)(((size_t)2 << 30) / ((size_t)(n * bins) * bins * sizeof(float))) / step * step;
+        if (slab < step) slab = step;
+        if (slab > round_up(n, step)) slab = round_up(n, step);
+        if ((rc = scratch(h, S_Q, q_bytes(slab), &q))) return rc;
+    }
+    const int64_t ldq = round_up(slab * bins, 128), lddw = round_up(m, 4);
+    void* dw;
+    if ((rc = scratch(h, S_DW, (size_t)(slab * bins * lddw) * sizeof(float), &dw))) return rc;
     CK(h, cudaMemsetAsync(wt, 0, (size_t)(m_pad * ldwt) * sizeof(float), h->stream), "memset weights");
+    if (rows) CK(h, cudaMemsetAsync(flag, 0, sizeof(int), h->stream), "memset flag");
     {
         PROF(h, "bspline_weights");
         CK(h, mcpg::launch_bspline_weights_fp32(X, n, m, ldx, bins, order, (float*)wt, ldwt, (double*)hd, h->stream,
                                                  &h->launches),
            "bspline weights kernel");
+        CK(h, mcpg::launch_bspline_weights_k32(X, n, m, ldx, bins, order, (float*)wk, ldk, h->stream, &h->launches),
+           "bspline weights kernel");
+        if (rows)
+            CK(h, mcpg::launch_mi_entries((const float*)wt, ldwt, genes, m, (float4*)ent, (int*)flag, h->stream,
+                                          &h->launches),
+               "weight entries kernel");
     }
     {
         PROF(h, "pair_sums");
         CK(h, mcpg::launch_pair_sums(G, ldg, n, (float*)gs, h->stream, &h->launches), "pair sums kernel");
     }
-    const int64_t T = (n + 15) / 16;
-    const int64_t ldq = ldwt;  // >= n*bins, multiple of 4
-    const size_t budget = (size_t)2 << 30;
-    int64_t tiles_per_slab = (int64_t)(budget / ((size_t)16 * bins * ldq * sizeof(float)));
-    if (tiles_per_slab < 1) tiles_per_slab = 1;
-    if (tiles_per_slab > T) tiles_per_slab = T;
-    const int64_t lddw = round_up(m, 4);
-    void *q, *dw;
-    if ((rc = scratch(h, S_Q, (size_t)(tiles_per_slab * 16 * bins * ldq) * sizeof(float), &q))) return rc;
-    if ((rc = scratch(h, S_DW, (size_t)(tiles_per_slab * 16 * bins * lddw) * sizeof(float), &dw))) return rc;
-    for (int64_t t0 = 0; t0 < T; t0 += tiles_per_slab) {
-        const int64_t nt = (t0 + tiles_per_slab <= T) ? tiles_per_slab : T - t0;
-        const int64_t g0 = t0 * 16, g1 = (g0 + nt * 16 < n) ? g0 + nt * 16 : n;
+    for (int64_t j0 = 0; j0 < n; j0 += slab) {
+        const int64_t j1 = std::min(j0 + slab, n);
         {
             PROF(h, "mi_q");
-            CK(h, mcpg::launch_mi_q((const float*)wt, ldwt, G, ldg, n, m, bins, t0, nt, (float*)q, ldq, h->stream,
-                                    &h->launches),
-               "MI adjoint Q kernel");
+            if (rows)
+                CK(h, mcpg::launch_mi_q_rows((const float*)wt, ldwt, (const float4*)ent, genes, (const int*)flag, G, ldg,
+                                             n, m, j0, j1, (float*)q, ldq, h->stream, &h->launches),
+                   "MI adjoint Q kernel");
+            else
+                CK(h, mcpg::launch_mi_q((const float*)wt, ldwt, G, ldg, n, m, bins, j0, j1, (float*)q, ldq, h->stream,
+                                        &h->launches),
+                   "MI adjoint Q kernel");
         }
-        mcpg::MaxminParams p{};
-        p.A = (const float*)q; p.lda = ldq; p.B = (const float*)wt; p.ldb = ldwt;
-        p.rows = (g1 - g0) * bins; p.cols = m; p.k_len = n * bins;
-        p.C = (float*)dw; p.ldc = lddw;
         {
             PROF(h, "gemm");
-            CK(h, mcpg::launch_maxmin(p, mcpg::MM_GEMM, 0, h->stream, &h->launches), "adjoint contraction kernel");
+            CK(h, mcpg::launch_gemm_fp32((const float*)q, ldq, (const float*)wk, ldk, (j1 - j0) * bins, m, n * bins,
+                                         (float*)dw, lddw, h->stream, &h->launches),
+               "adjoint contraction kernel");
         }
         {
             PROF(h, "mi_bwd_x");
-            CK(h, mcpg::launch_mi_bwd_x(X, n, m, ldx, bins, order, g0, g1, (const float*)gs, (const float*)dw, lddw,
+            CK(h, mcpg::launch_mi_bwd_x(X, n, m, ldx, bins, order, j0, j1, (const float*)gs, (const float*)dw, lddw,
                                         dX, lddx, h->stream, &h->launches),
                "MI adjoint x kernel");
         }

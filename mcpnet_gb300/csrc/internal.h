@@ -17,7 +17,6 @@ enum MaxminMode : int {
     MM_EXCL = 4,     // C = max over admissible k of min(A[i][k], B[j][k]); k excluded as in
                      // MM_DPI; an output with no admissible k is NaN
     MM_WITNESS = 5,  // C = A (x) B and K[i][j] = first k attaining it (-1 where C is -inf)
-    MM_GEMM = 6,     // C = A B^T in (+, x): the plus-times twin of the kernel (FP32 FFMA)
     MM_DPI1 = 7,     // first phase of the two-phase DPI: k runs over [0, k_len) only; outputs it
                      // decides are written (as MM_DPI), the others appended to `pending`
 };
@@ -199,7 +198,19 @@ cudaError_t launch_mi_rows(const float* Wt, int64_t ldwt, const float4* ent, int
                            const double* H, int64_t n, int64_t m, float* MI, int64_t ldmi, int64_t gene0,
                            int64_t gene1, cudaStream_t stream, int64_t* launches);
 cudaError_t launch_mi_q(const float* Wt, int64_t ldwt, const float* G, int64_t ldg, int64_t n, int64_t m, int bins,
-                        int64_t tile0, int64_t tiles, float* Q, int64_t ldq, cudaStream_t stream, int64_t* launches);
+                        int64_t j0, int64_t j1, float* Q, int64_t ldq, cudaStream_t stream, int64_t* launches);
+// The same Q from the inputs of launch_mi_rows (j0 a multiple of 32); over all genes j, each
+// unordered pair is computed once and written twice.
+cudaError_t launch_mi_q_rows(const float* Wt, int64_t ldwt, const float4* ent, int64_t ldge, const int* irregular,
+                             const float* G, int64_t ldg, int64_t n, int64_t m, int64_t j0, int64_t j1, float* Q,
+                             int64_t ldq, cudaStream_t stream, int64_t* launches);
+// C[r][s] = sum_k A[k][r] B[k][s], k ascending in one FP32 multiply-add chain (gemm_fp32.cu).  lda, ldb
+// multiples of 128 and at least R and S rounded up to that.
+cudaError_t launch_gemm_fp32(const float* A, int64_t lda, const float* B, int64_t ldb, int64_t R, int64_t S, int64_t K,
+                             float* C, int64_t ldc, cudaStream_t stream, int64_t* launches);
+// FP32 weights gene-bin-major: W[(gene * bins + a) * ldw + s], zero for s in [m, ldw).
+cudaError_t launch_bspline_weights_k32(const float* X, int64_t n, int64_t m, int64_t ldx, int bins, int order, float* W,
+                                       int64_t ldw, cudaStream_t stream, int64_t* launches);
 // gsum[i] = sum_{j != i} (G[i][j] + G[j][i])
 cudaError_t launch_pair_sums(const float* G, int64_t ldg, int64_t n, float* gsum, cudaStream_t stream,
                              int64_t* launches);

@@ -130,8 +130,7 @@ __global__ void __launch_bounds__(THREADS, MCPG_MM_MINB) maxmin_kernel(const Max
     constexpr bool DPI1 = (MODE == MM_DPI1);
     constexpr bool EXCL = (MODE == MM_DPI || MODE == MM_EXCL || DPI1);
     constexpr bool WIT = (MODE == MM_WITNESS);
-    constexpr bool GEMM = (MODE == MM_GEMM);
-    const float init = EXCL ? __int_as_float(0x7fc00000) : (GEMM ? 0.0f : -INFINITY);
+    const float init = EXCL ? __int_as_float(0x7fc00000) : -INFINITY;
     int32_t kidx[WIT ? 8 : 1][WIT ? TN : 1];
     if (WIT) {
 #pragma unroll
@@ -191,7 +190,7 @@ __global__ void __launch_bounds__(THREADS, MCPG_MM_MINB) maxmin_kernel(const Max
                    (k0 < i0 + BM && k0 + BK > i0) || (k0 < j0 + BN && k0 + BK > j0);
         }
         if (kmax == BK && !excl) {
-            if (WIT || GEMM) {
+            if (WIT) {
 #pragma unroll
                 for (int kk = 0; kk < BK; kk += 4) {
                     float4 a[8];
@@ -202,21 +201,14 @@ __global__ void __launch_bounds__(THREADS, MCPG_MM_MINB) maxmin_kernel(const Max
                         const float4 b = *reinterpret_cast<const float4*>(b_base + r * TXS * LDS + kk);
 #pragma unroll
                         for (int q = 0; q < 8; ++q) {
-                            if (GEMM) {
-                                float t = fmaf(a[q].x, b.x, acc[q][r]);
-                                t = fmaf(a[q].y, b.y, t);
-                                t = fmaf(a[q].z, b.z, t);
-                                acc[q][r] = fmaf(a[q].w, b.w, t);
-                            } else {
-                                // first k attaining the running maximum (strict >)
-                                const int32_t y0 = (int32_t)(k0 + kk);
-                                const float v0 = fmin2(a[q].x, b.x), v1 = fmin2(a[q].y, b.y);
-                                const float v2 = fmin2(a[q].z, b.z), v3 = fmin2(a[q].w, b.w);
-                                if (v0 > acc[q][r]) { acc[q][r] = v0; kidx[WIT ? q : 0][WIT ? r : 0] = y0; }
-                                if (v1 > acc[q][r]) { acc[q][r] = v1; kidx[WIT ? q : 0][WIT ? r : 0] = y0 + 1; }
-                                if (v2 > acc[q][r]) { acc[q][r] = v2; kidx[WIT ? q : 0][WIT ? r : 0] = y0 + 2; }
-                                if (v3 > acc[q][r]) { acc[q][r] = v3; kidx[WIT ? q : 0][WIT ? r : 0] = y0 + 3; }
-                            }
+                            // first k attaining the running maximum (strict >)
+                            const int32_t y0 = (int32_t)(k0 + kk);
+                            const float v0 = fmin2(a[q].x, b.x), v1 = fmin2(a[q].y, b.y);
+                            const float v2 = fmin2(a[q].z, b.z), v3 = fmin2(a[q].w, b.w);
+                            if (v0 > acc[q][r]) { acc[q][r] = v0; kidx[WIT ? q : 0][WIT ? r : 0] = y0; }
+                            if (v1 > acc[q][r]) { acc[q][r] = v1; kidx[WIT ? q : 0][WIT ? r : 0] = y0 + 1; }
+                            if (v2 > acc[q][r]) { acc[q][r] = v2; kidx[WIT ? q : 0][WIT ? r : 0] = y0 + 2; }
+                            if (v3 > acc[q][r]) { acc[q][r] = v3; kidx[WIT ? q : 0][WIT ? r : 0] = y0 + 3; }
                         }
                     }
                 }
@@ -263,10 +255,6 @@ __global__ void __launch_bounds__(THREADS, MCPG_MM_MINB) maxmin_kernel(const Max
                 for (int q = 0; q < 8; ++q)
 #pragma unroll
                     for (int r = 0; r < TN; ++r) {
-                        if (GEMM) {
-                            acc[q][r] = fmaf(a[q], b[r], acc[q][r]);
-                            continue;
-                        }
                         float v = fmin2(a[q], b[r]);
                         if (WIT) {
                             if (v > acc[q][r]) { acc[q][r] = v; kidx[WIT ? q : 0][WIT ? r : 0] = (int32_t)y; }
@@ -295,7 +283,7 @@ __global__ void __launch_bounds__(THREADS, MCPG_MM_MINB) maxmin_kernel(const Max
             const int64_t j = j0 + tx + TXS * r;
             if (j >= p.cols) continue;
             const float m = acc[q][r];
-            if (MODE == MM_PLAIN || MODE == MM_EXCL || MODE == MM_GEMM) {
+            if (MODE == MM_PLAIN || MODE == MM_EXCL) {
                 p.C[i * p.ldc + j] = m;
                 if (mirror) p.C[j * p.ldc + i] = m;
             } else if (MODE == MM_WITNESS) {
@@ -624,7 +612,6 @@ cudaError_t launch_maxmin(const MaxminParams& p, int mode, int symmetric, cudaSt
         case MM_EXCL: return s ? launch_one<MM_EXCL, true>(p, stream) : launch_one<MM_EXCL, false>(p, stream);
         case MM_WITNESS:
             return s ? launch_one<MM_WITNESS, true>(p, stream) : launch_one<MM_WITNESS, false>(p, stream);
-        case MM_GEMM: return launch_one<MM_GEMM, false>(p, stream);
         case MM_DPI1: return s ? launch_one<MM_DPI1, true>(p, stream) : launch_one<MM_DPI1, false>(p, stream);
         default: return cudaErrorInvalidValue;
     }

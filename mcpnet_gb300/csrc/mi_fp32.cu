@@ -49,13 +49,14 @@ __device__ __forceinline__ void tri_tile(int64_t b, int64_t T, int64_t& ti, int6
     tj = r + (b - (r * T - r * (r - 1) / 2));
 }
 
-// Adjoint epilogue arguments (EPI == 1): Q[(i - q_gene0) * BINS + a][j * BINS + b]
+// Adjoint epilogue arguments (EPI >= 1): Q[i * BINS + a][(j - j0) * BINS + b]
 // = Gs_ij (log2 P_ab + 1/ln 2) for P_ab > 0 (else 0), Gs_ij = G[i][j] + G[j][i]
-// for i != j and 0 on the diagonal; tiles cover A genes [16*q_tile0, ...) x all genes.
+// for i != j and 0 on the diagonal, for all genes i and the genes j in [j0, j1).  Q over all
+// genes is symmetric bit for bit (the sums' products commute).
 struct QArgs {
     const float* G; int64_t ldg;
     float* Q; int64_t ldq;
-    int64_t q_tile0;
+    int64_t j0, j1;
 };
 
 template <int BINS, int EPI>
@@ -71,8 +72,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (EPI == 0) {
         tri_tile(tile_base + blockIdx.x, T, ti, tj);
     } else {
-        ti = qa.q_tile0 + blockIdx.x / T;
-        tj = blockIdx.x % T;
+        const int64_t slab = (qa.j1 - qa.j0 + G - 1) / G;
+        ti = blockIdx.x / slab;
+        tj = qa.j0 / G + blockIdx.x % slab;
     }
     const int64_t gi0 = ti * G, gj0 = tj * G;
 
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (i >= n || j >= n) return;
         const float gs = (i == j) ? 0.0f : qa.G[i * qa.ldg + j] + qa.G[j * qa.ldg + i];
         const float c = 1.4426950408889634f;  // 1 / ln 2
-        float* Qr = qa.Q + (i - qa.q_tile0 * G) * BINS * qa.ldq + j * BINS;
+        float* Qr = qa.Q + i * BINS * qa.ldq + (j - qa.j0) * BINS;
 #pragma unroll
         for (int x = 0; x < BINS; ++x)
 #pragma unroll
@@ -278,8 +280,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     extern __shared__ float4 smem_f4[];
     float* smem = reinterpret_cast<float*>(smem_f4);
     // grid: 4 j tiles (fastest), i tiles, groups of 4 j tiles
-    const int64_t gi0 = i0 + (int64_t)blockIdx.y * WARPS, gj0 = ((int64_t)blockIdx.z * 4 + blockIdx.x) * SJ;
-    if (gj0 >= n || (EPI == 0 && gj0 + SJ <= gi0)) return;
+    const int64_t gi0 = i0 + (int64_t)blockIdx.y * WARPS, gj0 = ((int64_t)blockIdx.z * 4 + blockIdx.x) * SJ + (EPI == 1 ? qa.j0 : 0);
+    if (gj0 >= (EPI == 1 ? qa.j1 : n) || (EPI != 1 && gj0 + SJ <= gi0)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     // a warp copies whole samples: 80 chunks of j weights, then the entries
@@ -335,21 +337,32 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     cp_async_wait<0>();
 
     const int64_t i = gi0 + warp, j = gj0 + lane;
-    if (EPI == 1) {
-        if (i >= i1 || j >= n) return;
+    if (EPI >= 1) {
+        if (i >= i1 || j >= (EPI == 1 ? qa.j1 : n) || (EPI == 2 && j < i)) return;
         const float gs = (i == j) ? 0.0f : qa.G[i * qa.ldg + j] + qa.G[j * qa.ldg + i];
         const float c = 1.4426950408889634f;  // 1 / ln 2
-        float* Qr = qa.Q + (i - qa.q_tile0 * G) * SB * qa.ldq + j * SB;
+        float* Qr = qa.Q + i * SB * qa.ldq + (j - qa.j0) * SB;
+        float2 v[SB][SB / 2];
 #pragma unroll
         for (int x = 0; x < SB; ++x)
 #pragma unroll
             for (int y = 0; y < SB / 2; ++y) {
                 const float2 u = unpack2(acc[x][y]);
                 const float p0 = u.x * inv_m, p1 = u.y * inv_m;
-                *reinterpret_cast<float2*>(Qr + x * qa.ldq + 2 * y) =
-                    make_float2((gs != 0.0f && p0 > 0.0f) ? gs * (__log2f(p0) + c) : 0.0f,
-                                (gs != 0.0f && p1 > 0.0f) ? gs * (__log2f(p1) + c) : 0.0f);
+                v[x][y] = make_float2((gs != 0.0f && p0 > 0.0f) ? gs * (__log2f(p0) + c) : 0.0f,
+                                      (gs != 0.0f && p1 > 0.0f) ? gs * (__log2f(p1) + c) : 0.0f);
+                *reinterpret_cast<float2*>(Qr + x * qa.ldq + 2 * y) = v[x][y];
             }
+        if (EPI == 2 && i != j) {
+            float* Qm = qa.Q + j * SB * qa.ldq + i * SB;
+#pragma unroll
+            for (int y = 0; y < SB / 2; ++y)
+#pragma unroll
+                for (int x = 0; x < SB; x += 2) {
+                    *reinterpret_cast<float2*>(Qm + (2 * y) * qa.ldq + x) = make_float2(v[x][y].x, v[x + 1][y].x);
+                    *reinterpret_cast<float2*>(Qm + (2 * y + 1) * qa.ldq + x) = make_float2(v[x][y].y, v[x + 1][y].y);
+                }
+        }
         return;
     }
     if (i >= i1 || j >= n || j < i) return;
@@ -414,7 +427,7 @@ cudaError_t launch_rows_warps(const float* Wt, int64_t ldwt, const float4* ent, 
     auto kern = mi_rows_kernel<WARPS, EPI>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 grid(4, (unsigned)ceil_div(i1 - i0, WARPS), (unsigned)ceil_div(n, 4 * SJ));
+    dim3 grid(4, (unsigned)ceil_div(i1 - i0, WARPS), (unsigned)ceil_div(EPI == 1 ? qa.j1 - qa.j0 : n, 4 * SJ));
     kern<<<grid, WARPS * 32, smem, stream>>>(Wt, ldwt, ent, ldg, irregular, H, n, ceil_div(m, SCH) * SCH,
                                              1.0f / (float)m, MI, ldmi, i0, i1, qa);
     return cudaGetLastError();
@@ -429,8 +442,9 @@ cudaError_t launch_rows(const float* Wt, int64_t ldwt, const float4* ent, int64_
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t jt = ceil_div(n, SJ), pairs = EPI == 0 ? 2 : 1;  // EPI 0: about half of the tiles hold some j >= i
-    auto tiles = [&](int64_t w) { return ceil_div(i1 - i0, w) * jt / pairs; };
+    const int64_t jt = ceil_div(EPI == 1 ? qa.j1 - qa.j0 : n, SJ);
+    // EPI 0, 2: about half of the tiles hold some j >= i
+    auto tiles = [&](int64_t w) { return ceil_div(i1 - i0, w) * jt / (EPI == 1 ? 1 : 2); };
     if (tiles(4) <= sms)
         return launch_rows_warps<4, EPI>(Wt, ldwt, ent, ldg, irregular, H, n, m, MI, ldmi, i0, i1, qa, stream);
     if (tiles(8) <= sms)
@@ -458,8 +472,7 @@ cudaError_t launch_bins(const float* Wt, int64_t ldwt, const double* H, int64_t 
 }
 
 template <int BINS>
-cudaError_t launch_q_bins(const float* Wt, int64_t ldwt, int64_t n, int64_t m, const QArgs& qa, int64_t tiles_a,
-                          cudaStream_t stream) {
+cudaError_t launch_q_bins(const float* Wt, int64_t ldwt, int64_t n, int64_t m, const QArgs& qa, cudaStream_t stream) {
     using C = MiCfg<BINS>;
     auto kern = mi_fp32_kernel<BINS, 1>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
@@ -467,8 +480,8 @@ cudaError_t launch_q_bins(const float* Wt, int64_t ldwt, int64_t n, int64_t m, c
     const int64_t T = ceil_div(n, G);
     const int64_t m_pad = ceil_div(m, BKS) * BKS;
     const float inv_m = 1.0f / (float)m;
-    kern<<<(unsigned)(tiles_a * T), THREADS, C::SMEM, stream>>>(Wt, ldwt, nullptr, n, m_pad, inv_m, nullptr, 0, T,
-                                                                qa, 0);
+    kern<<<(unsigned)(T * ceil_div(qa.j1 - qa.j0, G)), THREADS, C::SMEM, stream>>>(Wt, ldwt, nullptr, n, m_pad, inv_m,
+                                                                                   nullptr, 0, T, qa, 0);
     return cudaGetLastError();
 }
 
@@ -497,24 +510,37 @@ cudaError_t launch_mi_rows(const float* Wt, int64_t ldwt, const float4* ent, int
     return launch_rows<0>(Wt, ldwt, ent, ldg, irregular, H, n, m, MI, ldmi, gene0, gene1, QArgs{}, stream);
 }
 
-// Adjoint slab: Q for A genes [16*tile0, 16*(tile0 + tiles)) x all genes.
-cudaError_t launch_mi_q(const float* Wt, int64_t ldwt, const float* G, int64_t ldg, int64_t n, int64_t m, int bins,
-                        int64_t tile0, int64_t tiles, float* Q, int64_t ldq, cudaStream_t stream, int64_t* launches) {
-    if (n <= 0 || tiles <= 0) return cudaSuccess;
+cudaError_t launch_mi_q_rows(const float* Wt, int64_t ldwt, const float4* ent, int64_t ldge, const int* irregular,
+                             const float* G, int64_t ldg, int64_t n, int64_t m, int64_t j0, int64_t j1, float* Q,
+                             int64_t ldq, cudaStream_t stream, int64_t* launches) {
+    if (n <= 0 || j0 >= j1) return cudaSuccess;
+    if (ldge != mi_rows_genes(n) || ldwt < ldge * SB || j0 % SJ || j1 > n || ldq % 2) return cudaErrorInvalidValue;
     if (launches) ++*launches;
-    QArgs qa{G, ldg, Q, ldq, tile0};
+    const QArgs qa{G, ldg, Q, ldq, j0, j1};
+    if (j0 == 0 && j1 == n)
+        return launch_rows<2>(Wt, ldwt, ent, ldge, irregular, nullptr, n, m, nullptr, 0, 0, n, qa, stream);
+    return launch_rows<1>(Wt, ldwt, ent, ldge, irregular, nullptr, n, m, nullptr, 0, 0, n, qa, stream);
+}
+
+// Adjoint slab: Q for all genes i and the genes j in [j0, j1), j0 a multiple of 16.
+cudaError_t launch_mi_q(const float* Wt, int64_t ldwt, const float* G, int64_t ldg, int64_t n, int64_t m, int bins,
+                        int64_t j0, int64_t j1, float* Q, int64_t ldq, cudaStream_t stream, int64_t* launches) {
+    if (n <= 0 || j0 >= j1) return cudaSuccess;
+    if (j0 % 16 || j1 > n) return cudaErrorInvalidValue;
+    if (launches) ++*launches;
+    QArgs qa{G, ldg, Q, ldq, j0, j1};
     switch (bins) {
-        case 2: return launch_q_bins<2>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 3: return launch_q_bins<3>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 4: return launch_q_bins<4>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 5: return launch_q_bins<5>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 6: return launch_q_bins<6>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 7: return launch_q_bins<7>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 8: return launch_q_bins<8>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 9: return launch_q_bins<9>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 10: return launch_q_bins<10>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 11: return launch_q_bins<11>(Wt, ldwt, n, m, qa, tiles, stream);
-        case 12: return launch_q_bins<12>(Wt, ldwt, n, m, qa, tiles, stream);
+        case 2: return launch_q_bins<2>(Wt, ldwt, n, m, qa, stream);
+        case 3: return launch_q_bins<3>(Wt, ldwt, n, m, qa, stream);
+        case 4: return launch_q_bins<4>(Wt, ldwt, n, m, qa, stream);
+        case 5: return launch_q_bins<5>(Wt, ldwt, n, m, qa, stream);
+        case 6: return launch_q_bins<6>(Wt, ldwt, n, m, qa, stream);
+        case 7: return launch_q_bins<7>(Wt, ldwt, n, m, qa, stream);
+        case 8: return launch_q_bins<8>(Wt, ldwt, n, m, qa, stream);
+        case 9: return launch_q_bins<9>(Wt, ldwt, n, m, qa, stream);
+        case 10: return launch_q_bins<10>(Wt, ldwt, n, m, qa, stream);
+        case 11: return launch_q_bins<11>(Wt, ldwt, n, m, qa, stream);
+        case 12: return launch_q_bins<12>(Wt, ldwt, n, m, qa, stream);
         default: return cudaErrorNotSupported;
     }
 }
