@@ -105,13 +105,13 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     a.cols = (int)(swap ? p.rows : p.cols);
     a.k = (int)p.k_len;
     if (!q.built) {
-        CK(h, mcpg::launch_ranked_lists(a.O, a.ldo, a.owners, a.k, q.L, r.cnt, h->stream, &h->launches), "lists kernel");
+        CK(h, mcpg::launch_ranked_lists(a.O, a.ldo, a.owners, a.k, 0, q.L, r.cnt, h->stream, &h->launches), "lists kernel");
         if (symm) CK(h, mcpg::launch_ranked_order(q.L, a.owners, q.rank, q.perm, h->stream, &h->launches), "order kernel");
         q.built = true;
     }
     a.L = q.L;
     a.ldt = round_up(a.cols, 128);
-    CK(h, mcpg::launch_ranked_transpose(a.X, a.ldx, a.cols, a.k, symm ? q.perm : nullptr, r.XT, a.ldt, r.cnt, h->stream,
+    CK(h, mcpg::launch_ranked_transpose(a.X, a.ldx, a.cols, a.k, 0, symm ? q.perm : nullptr, r.XT, a.ldt, r.cnt, h->stream,
                                         &h->launches),
        "transpose kernel");
     a.XT = r.XT;
@@ -262,6 +262,38 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
     p.tol_mult = 1.0 / (1.0 - (double)tol);  // dpi_kernel ctor, dpi.hpp:47
     p.mask = mask; p.ldmask = n;
     p.removed = cnt_removed;
+    // Candidates in descending order (maxmin_ranked.cu); when that gives up, the forms below.
+    Ranked rk;
+    ranked_begin(h, rk, n, n, n, 1);
+    if (rk.on) {
+        RankedSet& q = rk.set[0];
+        mcpg::RankedArgs r{};
+        r.O = a; r.ldo = la; r.X = a; r.ldx = la;
+        r.owners = r.cols = r.k = (int)n;
+        r.L = q.L; r.perm = q.perm;
+        r.XT = rk.XT; r.ldt = round_up(n, 128);
+        r.P = rk.P; r.ldp = round_up(n, 128);
+        r.direct = r.mirror = 1;
+        r.pending = rk.pending; r.pending_cap = rk.cap;
+        r.nan = rk.cnt; r.pending_n = rk.cnt + 1;
+        unsigned long long* gone = rk.cnt + 2;
+        {
+            PROF(h, "dpi");
+            CK(h, mcpg::launch_ranked_lists(a, la, n, n, 1, q.L, rk.cnt, h->stream, &h->launches), "lists kernel");
+            CK(h, mcpg::launch_ranked_order(q.L, n, q.rank, q.perm, h->stream, &h->launches), "order kernel");
+            CK(h, mcpg::launch_ranked_transpose(a, la, n, n, 1, q.perm, rk.XT, r.ldt, rk.cnt, h->stream, &h->launches),
+               "transpose kernel");
+            CK(h, mcpg::launch_ranked_dpi(r, q.rank, p.tol_mult, out, ldo, mask, n, gone, h->stream, &h->launches),
+               "ranked DPI kernels");
+        }
+        unsigned long long got[3] = {0, 0, 0};  // NaN seen, pending, removed
+        CK(h, cudaMemcpyAsync(got, rk.cnt, sizeof got, cudaMemcpyDeviceToHost, h->stream), "read counters");
+        CK(h, cudaStreamSynchronize(h->stream), "stream synchronize");
+        if (got[0] == 0 && got[1] <= (unsigned long long)rk.cap) {
+            if (removed) *removed = (int64_t)got[2];
+            return MCPG_OK;
+        }
+    }
     // Two phases for larger matrices: the tiled max-min over the first DPI_K0
     // intermediates decides most outputs (on MI matrices ~98 % are deleted by then);
     // the rest continue the scan one warp per output pair with the reference's early

@@ -92,14 +92,21 @@ struct RankedArgs {
     const unsigned long long* nan;  // nonzero: an operand holds a NaN, and it gave up too
 };
 int ranked_list_cap(int64_t k);
-cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64_t k, const RankedLists& L,
+// skip_diag: entry (i, i) is not listed / -inf in XT
+cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64_t k, int skip_diag, const RankedLists& L,
                                 unsigned long long* nan, cudaStream_t st, int64_t* launches);
 cudaError_t launch_ranked_order(const RankedLists& L, int64_t n, int* rank, int* perm, cudaStream_t st,
                                 int64_t* launches);
-cudaError_t launch_ranked_transpose(const float* X, int64_t ldx, int64_t rows, int64_t k, const int* perm, float* XT,
+cudaError_t launch_ranked_transpose(const float* X, int64_t ldx, int64_t rows, int64_t k, int skip_diag,
+                                    const int* perm, float* XT,
                                     int64_t ldt, unsigned long long* nan, cudaStream_t st, int64_t* launches);
 // symmetric: O == X, owners in the order of perm, only columns at or after the owner.
 cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t st, int64_t* launches);
+// The DPI filter of O == X (lists and XT with skip_diag): out / mask in gene order, *removed += the
+// entries that changed; nothing when the ranked form gave up.
+cudaError_t launch_ranked_dpi(const RankedArgs& a, const int* rank, double tol_mult, float* out, int64_t ldo,
+                              uint8_t* mask, int64_t ldmask, unsigned long long* removed, cudaStream_t st,
+                              int64_t* launches);
 // C[i][j] = P[rrank ? rrank[i] : i][crank ? crank[j] : j] and R = ratio(E, C), each nullable;
 // nothing when the ranked form gave up.
 cudaError_t launch_ranked_finish(const RankedArgs& a, const int* rrank, const int* crank, int64_t rows, int64_t cols,

@@ -120,3 +120,39 @@ def test_products_under_stream_capture(built_lib, warm):
             assert np.array_equal(bits(C.cpu().numpy()), bits(exhaustive(a, a)))
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("n,tol", [(256, 0.1), (301, 0.0), (517, 0.15), (300, 1.0)])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_dpi_equals_the_reference_loop(gpu, port, kind, n, tol, symmetric):
+    rng = np.random.default_rng(n + KINDS.index(kind))
+    A = data(kind, n, n, rng)
+    if symmetric:
+        A = np.maximum(A, A.T)
+    with np.errstate(all="ignore"):
+        out, mask, removed = gpu.dpi(A, tol, want_mask=True)
+        oo, om, orem = port.dpi(A, tol)
+    # at tol = 1 a zero entry's threshold is 0 * inf = NaN: the library keeps such an entry (as its product form
+    # does), the reference's loop clears it; it is a zero of either sign in both
+    defined = slice(None) if tol < 1.0 else A != 0.0
+    assert np.array_equal(mask[defined], om[defined])
+    assert np.array_equal(bits(out)[defined], bits(oo)[defined])
+    assert removed == orem
+
+
+def test_dpi_on_a_nan_matrix_takes_the_product_form(gpu):
+    """The deletions of a matrix with NaN entries outside some pairs' rows: those pairs decide as without."""
+    rng = np.random.default_rng(2)
+    n = 300
+    A = data("skewed", n, n, rng)
+    A = np.maximum(A, A.T)
+    B = np.zeros((n + 1, n + 1), np.float32)
+    B[:n, :n] = A
+    B[n, 1:n:2] = B[1:n:2, n] = np.nan
+    clean, cmask, _ = gpu.dpi(A, 0.1, want_mask=True)
+    out, mask, _ = gpu.dpi(B, 0.1, want_mask=True)
+    even = np.arange(0, n, 2)  # rows without a NaN: the extra gene adds min(0, 0) as a candidate only
+    pos = A[np.ix_(even, even)] > 0
+    assert np.array_equal(mask[np.ix_(even, even)][pos], cmask[np.ix_(even, even)][pos])
+    assert np.array_equal(out[np.ix_(even, even)][pos], clean[np.ix_(even, even)][pos])
