@@ -25,7 +25,6 @@ struct RankedSet {
 // The scratch of one API call's ranked products.
 struct Ranked {
     bool on = false;
-    int64_t owners = 0, cols = 0, k = 0;  // largest of the call's products
     float *XT = nullptr, *P = nullptr;
     mcpg::RankedPending* pending = nullptr;
     int64_t cap = 0;
@@ -35,22 +34,22 @@ struct Ranked {
 };
 constexpr int RANKED_COUNTERS = 8;
 
-// Decides whether this call's products take the ranked form, and lays out its scratch.  Dense below
+// Decides whether this call's products (at most rows x cols over k) take the ranked form, and lays out
+// its scratch.  Dense below
 // MCPG_RANKED_MIN candidates or rows (the ranked form's six launches cost more than one small
 // product), above the list kernel's 32,768 candidates or the finishing kernel's row buffer, where
 // the scratch cannot be had, and in a stream capture that would have to allocate it.
-void ranked_begin(mcpg_handle* h, Ranked& r, int64_t owners, int64_t cols, int64_t k, int lists) {
+void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t k, int lists) {
     r = Ranked{};
-    if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || owners < 8 || k > 32768 || owners > 50000 || cols > 50000) return;
-    const int64_t lx = round_up(std::max(owners, cols), 128);
-    const int64_t rows = std::max(owners, cols);
+    if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || rows < 8 || k > 32768 || rows > 50000 || cols > 50000) return;
+    const int64_t most = std::max(rows, cols), lx = round_up(most, 128);  // either operand may own the lists
     const int64_t pitch = mcpg::ranked_list_cap(k);
-    r.cap = std::max<int64_t>(4096, owners * cols / 64);
-    const size_t lbytes = (size_t)rows * (size_t)pitch * sizeof(uint2) + (size_t)rows * 5 * sizeof(int);
+    r.cap = std::max<int64_t>(4096, rows * cols / 64);
+    const size_t lbytes = (size_t)most * (size_t)pitch * sizeof(uint2) + (size_t)most * 5 * sizeof(int);
     struct { int slot; size_t bytes; void* p; } need[] = {
         {S_RK_CNT, RANKED_COUNTERS * sizeof(unsigned long long), nullptr},
         {S_RK_XT, (size_t)k * (size_t)lx * sizeof(float), nullptr},
-        {S_RK_P, (size_t)rows * (size_t)lx * sizeof(float), nullptr},
+        {S_RK_P, (size_t)rows * (size_t)round_up(cols, 128) * sizeof(float), nullptr},
         {S_RK_PEND, (size_t)r.cap * sizeof(mcpg::RankedPending), nullptr},
         {S_RK_L0, lbytes, nullptr},
         {S_RK_L1, lists > 1 ? lbytes : 0, nullptr},
@@ -75,15 +74,14 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t owners, int64_t cols, int64
         char* p = (char*)need[4 + s].p;
         q.L.entries = (uint2*)p;
         q.L.pitch = pitch;
-        p += (size_t)rows * (size_t)pitch * sizeof(uint2);
+        p += (size_t)most * (size_t)pitch * sizeof(uint2);
         q.L.count = (int*)p;
-        q.L.bound = (float*)(q.L.count + rows);
-        q.L.strength = (int*)(q.L.bound + rows);
-        q.rank = q.L.strength + rows;
-        q.perm = q.rank + rows;
+        q.L.bound = (float*)(q.L.count + most);
+        q.L.strength = (int*)(q.L.bound + most);
+        q.rank = q.L.strength + most;
+        q.perm = q.rank + most;
     }
     if (cudaMemsetAsync(r.cnt, 0, RANKED_COUNTERS * sizeof(unsigned long long), h->stream) != cudaSuccess) return;
-    r.owners = owners; r.cols = cols; r.k = k;
     r.on = true;
 }
 
@@ -423,12 +421,9 @@ int maxmin_masked_dev(mcpg_handle* h, const float* A, int64_t lda, const float* 
         if ((rc = aligned_view(h, B, ldb, cols, k, S_TFB, &bb, &lb))) return rc;
         p.A = (const float*)a; p.lda = ldk; p.B = bb; p.ldb = lb; p.k_len = k;
     }
-    {
-        PROF(h, "maxmin");
-        CK(h, mcpg::launch_maxmin(p, mcpg::MM_PLAIN, (same && ts.pm_inf) ? 1 : 0, h->stream, &h->launches),
-           "maxmin kernel");
-    }
-    return MCPG_OK;
+    Ranked r;
+    ranked_begin(h, r, rows, cols, p.k_len, 1);
+    return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, same && ts.pm_inf, false);
 }
 
 // compute_mcp{2,3,4}_tfs (mcpnet_helper.hpp:209-243, 281-333, 367-434):
@@ -518,6 +513,48 @@ int maxmins_tf_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, const
     const float* TG = (const float*)tg;
     if (T_out) CK(h, mcpg::launch_copy2d(TG, ldt, T_out, ldto, t, n, h->stream), "copy2d");
     if (!M1 && !M2 && !M3) return MCPG_OK;
+    if (ts.pm_inf) {
+        // A pure TF mask leaves the TF columns: products over t candidates, with A's gathered once.
+        // (A (x)m A)[j][k] for a TF k is max_l min(A[j][l], A[k][l]) over the TFs l: M1[k][j].  So
+        // M3's second operand is M1 transposed, and the n x n product is not formed.
+        const int64_t lk = round_up(t, 128);
+        void *ag, *tt, *mt = nullptr, *m1p = M1, *nan;
+        if ((rc = scratch(h, S_TFB, (size_t)(n * lk) * sizeof(float), &ag))) return rc;
+        if ((rc = scratch(h, S_TFA, (size_t)(t * lk) * sizeof(float), &tt))) return rc;
+        if (!M1 && (rc = scratch(h, S_M3, (size_t)(t * ldt) * sizeof(float), &m1p))) return rc;
+        if (M3 && (rc = scratch(h, S_M1, (size_t)(n * lk) * sizeof(float), &mt))) return rc;
+        if ((rc = scratch(h, S_SMALL, 64, &nan))) return rc;
+        const int64_t l1p = M1 ? ld1 : ldt;
+        CK(h, mcpg::launch_gather(A, lda, nullptr, (const int*)idx, n, t, (float*)ag, lk, h->stream, &h->launches),
+           "gather kernel");
+        CK(h, mcpg::launch_gather(TG, ldt, nullptr, (const int*)idx, t, t, (float*)tt, lk, h->stream, &h->launches),
+           "gather kernel");
+        Ranked rk;
+        ranked_begin(h, rk, t, n, t, 2);
+        mcpg::MaxminParams p{};
+        p.rows = t; p.cols = n; p.k_len = t;
+        p.A = (const float*)tt; p.lda = lk; p.B = (const float*)ag; p.ldb = lk;
+        p.C = (float*)m1p; p.ldc = l1p;
+        if ((rc = ranked_product(h, rk, 0, p, mcpg::MM_PLAIN, false, false))) return rc;  // ttg
+        if (!M2 && !M3) return MCPG_OK;
+        rk.set[0].built = false;  // M1's TF columns take T's place
+        CK(h, mcpg::launch_gather((const float*)m1p, l1p, nullptr, (const int*)idx, t, t, (float*)tt, lk, h->stream,
+                                  &h->launches),
+           "gather kernel");
+        if (M2) {  // A's rows own the lists: M1's have no pronounced largest values
+            p.C = M2; p.ldc = ld2;
+            if ((rc = ranked_product(h, rk, 1, p, mcpg::MM_PLAIN, false, true))) return rc;  // tttg
+        }
+        if (M3) {
+            CK(h, mcpg::launch_ranked_transpose((const float*)m1p, l1p, t, n, 0, nullptr, (float*)mt, lk,
+                                                (unsigned long long*)nan, h->stream, &h->launches),
+               "transpose kernel");
+            p.B = (const float*)mt;
+            p.C = M3; p.ldc = ld3;
+            if ((rc = ranked_product(h, rk, 0, p, mcpg::MM_PLAIN, false, false))) return rc;  // ttttg
+        }
+        return MCPG_OK;
+    }
     float* m1 = M1;
     int64_t l1 = ld1;
     if (!m1) {
