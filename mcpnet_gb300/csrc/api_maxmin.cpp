@@ -26,6 +26,7 @@ struct RankedSet {
 struct Ranked {
     bool on = false;
     float *XT = nullptr, *P = nullptr;
+    int* PK = nullptr;
     mcpg::RankedPending* pending = nullptr;
     int64_t cap = 0;
     unsigned long long* cnt = nullptr;  // [0]: NaN seen, [1..]: a pending count per product
@@ -39,7 +40,7 @@ constexpr int RANKED_COUNTERS = 8;
 // MCPG_RANKED_MIN candidates or rows (the ranked form's six launches cost more than one small
 // product), above the list kernel's 32,768 candidates or the finishing kernel's row buffer, where
 // the scratch cannot be had, and in a stream capture that would have to allocate it.
-void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t k, int lists) {
+void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t k, int lists, bool witness = false) {
     r = Ranked{};
     if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || rows < 8 || k > 32768 || rows > 50000 || cols > 50000) return;
     const int64_t most = std::max(rows, cols), lx = round_up(most, 128);  // either operand may own the lists
@@ -53,6 +54,7 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
         {S_RK_PEND, (size_t)r.cap * sizeof(mcpg::RankedPending), nullptr},
         {S_RK_L0, lbytes, nullptr},
         {S_RK_L1, lists > 1 ? lbytes : 0, nullptr},
+        {S_RK_K, witness ? (size_t)rows * (size_t)round_up(cols, 128) * sizeof(int) : 0, nullptr},
     };
     bool grow = false;
     for (auto& q : need) grow |= q.bytes > h->cap[q.slot];
@@ -69,6 +71,7 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
     r.XT = (float*)need[1].p;
     r.P = (float*)need[2].p;
     r.pending = (mcpg::RankedPending*)need[3].p;
+    r.PK = (int*)need[6].p;
     for (int s = 0; s < lists; ++s) {
         RankedSet& q = r.set[s];
         char* p = (char*)need[4 + s].p;
@@ -90,11 +93,11 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
 // pronounced largest values.  Falls back to the exhaustive kernel on the device.
 int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p, int mode, bool symm, bool swap) {
     if (!r.on || r.used >= RANKED_COUNTERS) {
-        PROF(h, "maxmin");
+        PROF(h, mode == mcpg::MM_WITNESS ? "maxmin_witness" : "maxmin");
         CK(h, mcpg::launch_maxmin(p, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
         return MCPG_OK;
     }
-    PROF(h, "maxmin");
+    PROF(h, mode == mcpg::MM_WITNESS ? "maxmin_witness" : "maxmin");
     RankedSet& q = r.set[s];
     mcpg::RankedArgs a{};
     a.O = swap ? p.B : p.A; a.ldo = swap ? p.ldb : p.lda;
@@ -124,6 +127,15 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     CK(h, mcpg::launch_ranked_walk(a, symm ? 1 : 0, h->stream, &h->launches), "ranked max-min kernel");
     mcpg::MaxminParams d = p;
     d.run_above = a.pending_n; d.run_cap = (unsigned long long)a.pending_cap; d.run_nan = a.nan;
+    if (mode == mcpg::MM_WITNESS) {
+        unsigned long long* open_n = r.cnt + r.used++;
+        d.run_above2 = open_n;
+        CK(h, mcpg::launch_ranked_witness(a, symm ? 1 : 0, q.rank, r.PK, open_n, p.rows, p.cols, p.C, p.ldc, p.K, p.ldk,
+                                          h->stream, &h->launches),
+           "ranked witness kernels");
+        CK(h, mcpg::launch_maxmin(d, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
+        return MCPG_OK;
+    }
     CK(h, mcpg::launch_maxmin(d, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
     CK(h, mcpg::launch_ranked_finish(a, symm ? q.rank : nullptr, symm ? q.rank : nullptr, p.rows, p.cols, p.C, p.ldc,
                                      p.E, p.lde, mode == mcpg::MM_RATIO ? p.R : nullptr, p.ldr, h->stream, &h->launches),
@@ -738,9 +750,9 @@ int maxmin_witness_dev(mcpg_handle* h, const float* A, int64_t lda, const float*
     mcpg::MaxminParams p{};
     p.A = a; p.lda = la; p.B = b; p.ldb = lb; p.rows = rows; p.cols = cols; p.k_len = k;
     p.C = C; p.ldc = ldc; p.K = K; p.ldk = ldk;
-    PROF(h, "maxmin_witness");
-    CK(h, mcpg::launch_maxmin(p, mcpg::MM_WITNESS, symm ? 1 : 0, h->stream, &h->launches), "maxmin witness kernel");
-    return MCPG_OK;
+    Ranked r;
+    ranked_begin(h, r, rows, cols, k, 1, true);
+    return ranked_product(h, r, 0, p, mcpg::MM_WITNESS, symm, false);
 }
 
 int maxmin_bwd_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb, int64_t rows,

@@ -56,9 +56,11 @@ struct MaxminParams {
     // MM_DPI / MM_DPI1 on a permuted input P A P^T: output (i, j) goes to
     // C / mask [perm[i]][perm[j]] (device, nullable = identity)
     const int* perm;
-    // run only when *run_above (device) exceeds run_cap or *run_nan is set (nullable: always run)
+    // run only when *run_above or *run_above2 (device) exceeds run_cap or *run_nan is set (run_above nullable:
+    // always run; run_above2 nullable)
     const unsigned long long* run_above; unsigned long long run_cap;
     const unsigned long long* run_nan;
+    const unsigned long long* run_above2;
 };
 
 // symmetric != 0: A == B (same rows), rows == cols; only tiles on or above the
@@ -107,6 +109,11 @@ cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t 
 cudaError_t launch_ranked_dpi(const RankedArgs& a, const int* rank, double tol_mult, float* out, int64_t ldo,
                               uint8_t* mask, int64_t ldmask, unsigned long long* removed, cudaStream_t st,
                               int64_t* launches);
+// C and the first k attaining it (as MM_WITNESS) after launch_ranked_walk; PK: as P, open_n: a zeroed count
+// (above pending_cap: gave up, and nothing is written).
+cudaError_t launch_ranked_witness(const RankedArgs& a, int symmetric, const int* rank, int* PK,
+                                  unsigned long long* open_n, int64_t rows, int64_t cols, float* C, int64_t ldc,
+                                  int32_t* K, int64_t ldk, cudaStream_t st, int64_t* launches);
 // C[i][j] = P[rrank ? rrank[i] : i][crank ? crank[j] : j] and R = ratio(E, C), each nullable;
 // nothing when the ranked form gave up.
 cudaError_t launch_ranked_finish(const RankedArgs& a, const int* rrank, const int* crank, int64_t rows, int64_t cols,

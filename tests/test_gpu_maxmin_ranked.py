@@ -156,3 +156,19 @@ def test_dpi_on_a_nan_matrix_takes_the_product_form(gpu):
     pos = A[np.ix_(even, even)] > 0
     assert np.array_equal(mask[np.ix_(even, even)][pos], cmask[np.ix_(even, even)][pos])
     assert np.array_equal(out[np.ix_(even, even)][pos], clean[np.ix_(even, even)][pos])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("rows,cols,k", [(256, 256, 256), (301, 260, 517), (8, 300, 1030)])
+def test_witnesses_equal_the_first_attaining_candidate(gpu, kind, rows, cols, k):
+    rng = np.random.default_rng(rows + k + KINDS.index(kind))
+    A, B = data(kind, rows, k, rng), data(kind, cols, k, rng)
+    for X, Y, args in ((A, B, (A, B)), (B, B, (B,))):
+        C, K = gpu.maxmin_witness(*args)
+        for i in range(X.shape[0]):
+            v = np.minimum(X[i][None, :], Y)
+            first = v.argmax(1)  # the first of equal values
+            value = v[np.arange(Y.shape[0]), first]
+            want = np.where(value == -np.inf, -1, first)
+            assert np.array_equal(K[i], want), i
+            assert np.array_equal(C[i], value), i
