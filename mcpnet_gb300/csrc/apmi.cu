@@ -12,21 +12,29 @@
 // (uint16; cH[k] = samples with rank < k).  m <= 16384.
 //
 // ap_mi_kernel: persistent blocks take the next X gene i from a global
-// counter; X's ranks sit in shared memory; each warp takes the next Y gene
-// j >= i and walks the reference's window quadtree for the pair:
-//   * x ranks grouped by y rank: xg[k] = xr[order_Y[k]] (warp-private shared)
-//   * a window's four sub-window counts come from one warp-strided scan of
-//     its y band, reduced with redux.sync
+// counter; X's ranks sit in shared memory, each with its quartile of the rank range;
+// each warp takes the next Y gene j >= i:
+//   * one pass over the samples in y-rank order counts the 4 x 4 grid of x and y quartiles (packed
+//     byte counters).  That decides the root window (always split) and its four children, which for
+//     unrelated genes is all: no grouped copy of the ranks, no further scan.
+//   * a child that splits again is walked as the reference's window quadtree: x ranks
+//     grouped by y rank, xg[k] = xr[order_Y[k]] (warp-private shared), and a window's
+//     four sub-window counts from one warp-strided scan of its y band
 //   * the chi-square split test `fl(S / e) > 7.815` is decided exactly in
 //     128-bit integers (S and e are exact in double, so only the rounding of
 //     the quotient matters, and it is reproduced against the midpoint of
 //     7.815 and its successor)
 //   * the depth-first order of the reference (a LIFO of pushed windows) is
-//     kept, leaves are queued in that order; 32 queued leaves are evaluated
-//     one per lane (nxy * log2(nxy / (nx*ny)) in double) and added to the sum
-//     in queue order, so the sum has the reference's order.
+//     kept; leaves are queued in that order, over several genes j, and
+//     evaluated 32 at a time, one per lane (nxy * log2(nxy / (nx*ny)) in double).  A lane
+//     then adds up one pair's leaves in queue order, so every sum has the reference's order.
+// FP64 is a narrow pipe here (a warp instruction takes 16 clocks of an SM, however few lanes are
+// active) and bound the kernel when every pair evaluated its own four-odd leaves and sums.
 // The only source of difference from the reference is log2 (CUDA's vs the
 // C library's, each within an ulp).
+// Measured (4,096 x 1,024 / 20,000 x 2,000): 28.8 / 879 ms when every pair scanned the root and its children one
+// by one and evaluated its own leaves, 8.9 / 359 ms now; at 64 registers (4 blocks per SM: instruction
+// fetch and latencies bound it; 80 registers and 3 blocks ran 9.9 / 451 ms).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -39,7 +47,7 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int AP_MAX_M = 16384;
 constexpr int AP_STACK = 64;   // the LIFO holds at most 3 * depth + 1 <= 46 windows for m <= 16384
-constexpr int AP_LEAVES = 32;
+constexpr int AP_LEAVES = 40;   // queue: flushed from 32 on, a step queues at most 4 more
 constexpr int AP_WARPS = 8;
 
 __device__ __forceinline__ uint32_t order_key_desc(float f) {
@@ -173,16 +181,15 @@ struct ApWin {
     uint32_t npts;
 };
 
-// fl((sum_q (c_q - n/4)^2) / (n/4)) > 7.815 in IEEE double, decided exactly:
-// with A = sum_q (4 c_q - n)^2 the quotient is A / (4n); 7.815 = K * 2^-50 and
-// the rounding boundary above it is (2K + 1) * 2^-51 (K odd: a tie rounds up).
+// fl((sum_q (c_q - n/4)^2) / (n/4)) > 7.815 in IEEE double, decided exactly for n = sum_q c_q <= 16384:
+// with A = sum_q (4 c_q - n)^2 = 16 sum_q c_q^2 - 4 n^2 (< 2^32) the quotient is A / (4n); 7.815 =
+// K * 2^-50 and the rounding boundary above it is (2K + 1) * 2^-51, so the test is A * 2^49 > (2K + 1) n
+// (never equal: 2K + 1 is odd and n < 2^49), that is A > floor((2K + 1) n / 2^49).
 __device__ __forceinline__ bool chi_square_above(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t n) {
-    const long long d0 = 4ll * c0 - n, d1 = 4ll * c1 - n, d2 = 4ll * c2 - n, d3 = 4ll * c3 - n;
-    const unsigned long long A = (unsigned long long)(d0 * d0 + d1 * d1 + d2 * d2 + d3 * d3);
-    constexpr unsigned long long K = 8798907771975107ull;  // 7.815 * 2^50, exact
-    const unsigned __int128 lhs = (unsigned __int128)A << 49;
-    const unsigned __int128 rhs = (unsigned __int128)(2 * K + 1) * n;
-    return lhs > rhs || (lhs == rhs && (K & 1));
+    constexpr unsigned long long B = 2 * 8798907771975107ull + 1;  // K = 7.815 * 2^50, exact
+    const uint32_t A = 16u * (c0 * c0 + c1 * c1 + c2 * c2 + c3 * c3) - 4u * n * n;
+    const unsigned long long t = (B >> 32) * n + (((B & 0xffffffffull) * n) >> 32);
+    return A > (uint32_t)(t >> 17);
 }
 
 struct ApArgs {
@@ -198,33 +205,48 @@ struct ApArgs {
     int warp_bytes;  // shared bytes per warp
 };
 
-__device__ __forceinline__ void ap_flush(const uint32_t* lnxy, const uint32_t* lnxny, int& nleaf, double& mi,
-                                         int lane) {
+// A warp's leaf queue over up to 32 pairs: lane s holds pair slot s, its running sum and its leaves' range
+// [beg, end) in the queue.  Evaluates all n <= AP_LEAVES queued leaves and adds each lane's range to sum, in
+// queue order.  Not inlined: the instructions of the double logarithm, at each place that queues leaves,
+// are more than the instruction cache holds.
+__device__ __noinline__ double ap_flush(const uint32_t* nxy, const uint32_t* nxny, double* term, int n, int beg,
+                                        int end, double sum) {
     __syncwarp();
-    double t = 0.0;
-    if (lane < nleaf) {
-        const double nxy = (double)lnxy[lane];
-        t = nxy * log2(nxy / (double)lnxny[lane]);
+    for (int k = threadIdx.x & 31; k < n; k += 32) {
+        const double c = (double)nxy[k];
+        term[k] = c * log2(c / (double)nxny[k]);
     }
-    for (int k = 0; k < nleaf; ++k) mi += __shfl_sync(FULL, t, k);  // queue order = the reference's order
-    nleaf = 0;
     __syncwarp();
+    const int most = (int)__reduce_max_sync(FULL, (unsigned)(end - beg));
+    for (int r = 0; r < most; ++r)
+        if (beg + r < end) sum += term[beg + r];
+    __syncwarp();
+    return sum;
 }
 
-__global__ void __launch_bounds__(AP_WARPS * 32) ap_mi_kernel(ApArgs a) {
+__global__ void __launch_bounds__(AP_WARPS * 32, 4) ap_mi_kernel(ApArgs a) {
     extern __shared__ __align__(16) unsigned char ap_smem[];
     __shared__ int s_i;
     __shared__ int s_next_j;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int m = (int)a.m;
     const int xr_bytes = (int)(((int64_t)m * 2 + 15) / 16 * 16);
-    uint16_t* xr = (uint16_t*)ap_smem;
+    uint16_t* xr = (uint16_t*)ap_smem;  // rank | quartile << 14
     unsigned char* wbase = ap_smem + xr_bytes + w * a.warp_bytes;
     ApWin* stack = (ApWin*)wbase;
-    uint32_t* lnxy = (uint32_t*)(wbase + AP_STACK * sizeof(ApWin));
+    double* term = (double*)(wbase + AP_STACK * sizeof(ApWin));
+    uint32_t* lnxy = (uint32_t*)(term + AP_LEAVES);
     uint32_t* lnxny = lnxy + AP_LEAVES;
     uint16_t* xg = (uint16_t*)(lnxny + AP_LEAVES);
+    int nq = 0, beg = 0, end = 0;  // queued leaves; this lane's slot's range
+    double sum = 0.0;
+    auto flush = [&]() {
+        sum = ap_flush(lnxy, lnxny, term, nq, beg, end, sum);
+        beg = end = nq = 0;
+    };
     const double logm = log2((double)m);
+    // the grid's boundaries: the midpoints of the root window and of its children
+    const int half = m >> 1, lo4 = half >> 1, hi4 = (half + m) >> 1;
 
     for (;;) {
         if (threadIdx.x == 0) {
@@ -234,94 +256,208 @@ __global__ void __launch_bounds__(AP_WARPS * 32) ap_mi_kernel(ApArgs a) {
         __syncthreads();
         const int i = s_i;
         if (i >= a.n) break;
-        for (int s = threadIdx.x; s < m; s += blockDim.x) xr[s] = a.xr[(int64_t)i * m + s];
+        for (int s = threadIdx.x; s < m; s += blockDim.x) {
+            const int r = a.xr[(int64_t)i * m + s];
+            xr[s] = (uint16_t)(r | (((r >= lo4) + (r >= half) + (r >= hi4)) << 14));
+        }
         __syncthreads();
         const uint16_t* cX = a.cH + (int64_t)i * a.ldc;
-        for (;;) {
+        const int nx_lo = cX[half], nx_hi = (int)cX[m] - nx_lo;
+        int slot = 0, jmine = 0;
+        bool broken_mine = false;
+        bool more = true;
+        while (more) {
             int j = 0;
             if (lane == 0) j = atomicAdd(&s_next_j, 1);
             j = __shfl_sync(FULL, j, 0);
-            if (j >= a.n) break;
+            more = j < a.n;
+            if (slot == 32 || !more) {  // the batch's pairs are complete
+                flush();
+                if (lane < slot) {
+                    float v = (float)(sum / (double)m + logm);
+                    if (broken_mine) {
+                        v = __int_as_float(0x7fc00000);
+                        atomicOr(a.flag, 2);
+                    }
+                    a.MI[(int64_t)i * a.ldmi + jmine] = v;
+                    a.MI[(int64_t)jmine * a.ldmi + i] = v;
+                }
+                slot = 0;
+                if (!more) break;
+            }
+            if (lane == slot) {
+                sum = 0.0;
+                beg = end = nq;
+                jmine = j;
+                broken_mine = false;
+            }
             const uint16_t* oY = a.order + (int64_t)j * m;
             const uint16_t* cY = a.cH + (int64_t)j * a.ldc;
-            for (int k = lane; k < m; k += 32) xg[k] = xr[oY[k]];
-            if (lane == 0) stack[0] = ApWin{0, 0, (uint16_t)m, (uint16_t)m, (uint32_t)m};
-            __syncwarp();
-            int top = 1, nleaf = 0;
-            bool root = true, broken = false;
-            double mi = 0.0;
-            int64_t guard = 0;
-            while (top > 0) {
-                if (++guard > 16ll * m + 64) {  // cannot happen: every pushed window is smaller than its parent
-                    broken = true;
-                    break;
-                }
-                const ApWin wv = stack[top - 1];
-                __syncwarp();
-                const int mx = (wv.x1 + wv.x2) >> 1, my = (wv.y1 + wv.y2) >> 1;
-                const int b0 = cY[wv.y1], b1 = cY[my], b2 = cY[wv.y2];
-                uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0;
-                for (int k = b0 + lane; k < b1; k += 32) {
-                    const int x = xg[k];
-                    c0 += (x >= wv.x1 && x < mx);
-                    c1 += (x >= mx && x < wv.x2);
-                }
-                for (int k = b1 + lane; k < b2; k += 32) {
-                    const int x = xg[k];
-                    c2 += (x >= wv.x1 && x < mx);
-                    c3 += (x >= mx && x < wv.x2);
-                }
-                c0 = __reduce_add_sync(FULL, c0);
-                c1 = __reduce_add_sync(FULL, c1);
-                c2 = __reduce_add_sync(FULL, c2);
-                c3 = __reduce_add_sync(FULL, c3);
-                --top;
-                if (root || chi_square_above(c0, c1, c2, c3, wv.npts)) {
-                    const int sx1[4] = {wv.x1, mx, wv.x1, mx}, sx2[4] = {mx, wv.x2, mx, wv.x2};
-                    const int sy1[4] = {wv.y1, wv.y1, my, my}, sy2[4] = {my, my, wv.y2, wv.y2};
-                    const uint32_t cc[4] = {c0, c1, c2, c3};
+            // y boundaries as positions in rank order
+            int bnd = 0;
+            if (lane < 5) bnd = cY[lane == 0 ? 0 : lane == 1 ? lo4 : lane == 2 ? half : lane == 3 ? hi4 : m];
+            int bpos[5];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const bool split = ((sx1[q] + 1) < sx2[q] || (sy1[q] + 1) < sy2[q]) && cc[q] > 2;
-                        if (split) {
-                            if (top >= AP_STACK) {
-                                broken = true;
-                                continue;
-                            }
-                            if (lane == 0)
-                                stack[top] = ApWin{(uint16_t)sx1[q], (uint16_t)sy1[q], (uint16_t)sx2[q],
-                                                   (uint16_t)sy2[q], cc[q]};
-                            ++top;
-                        } else if (cc[q] > 0) {
-                            if (lane == 0) {
-                                lnxy[nleaf] = cc[q];
-                                lnxny[nleaf] = (uint32_t)(cX[sx2[q]] - cX[sx1[q]]) * (uint32_t)(cY[sy2[q]] - cY[sy1[q]]);
-                            }
-                            if (++nleaf == AP_LEAVES) ap_flush(lnxy, lnxny, nleaf, mi, lane);
-                        }
+            for (int e = 0; e < 5; ++e) bpos[e] = __shfl_sync(FULL, bnd, e);
+            uint32_t g[4][4];  // [y quartile][x quartile]
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                uint32_t acc = 0;  // four byte counters: a lane sees at most ceil(m / 4 / 32) + ties <= 255 samples
+                uint32_t wide = 0, wide2 = 0;
+                int k = bpos[e] + lane;
+                int left = 255;
+                for (; k + 96 < bpos[e + 1]; k += 128) {
+                    const uint32_t o0 = oY[k], o1 = oY[k + 32], o2 = oY[k + 64], o3 = oY[k + 96];
+                    const uint32_t v0 = xr[o0], v1 = xr[o1], v2 = xr[o2], v3 = xr[o3];
+                    acc += (1u << ((v0 >> 11) & 24u)) + (1u << ((v1 >> 11) & 24u));
+                    acc += (1u << ((v2 >> 11) & 24u)) + (1u << ((v3 >> 11) & 24u));
+                    left -= 4;
+                    if (left < 4) {  // widen before a byte can overflow
+                        wide += (acc & 0xffu) + ((acc & 0xff00u) << 8);
+                        wide2 += ((acc >> 16) & 0xffu) + ((acc >> 24) << 16);
+                        acc = 0;
+                        left = 255;
                     }
-                } else {
-                    if (lane == 0) {
-                        lnxy[nleaf] = wv.npts;
-                        lnxny[nleaf] = (uint32_t)(cX[wv.x2] - cX[wv.x1]) * (uint32_t)(cY[wv.y2] - cY[wv.y1]);
-                    }
-                    if (++nleaf == AP_LEAVES) ap_flush(lnxy, lnxny, nleaf, mi, lane);
                 }
-                root = false;
+                for (; k < bpos[e + 1]; k += 32) acc += 1u << (((uint32_t)xr[oY[k]] >> 11) & 24u);
+                wide += (acc & 0xffu) + ((acc & 0xff00u) << 8);
+                wide2 += ((acc >> 16) & 0xffu) + ((acc >> 24) << 16);
+                wide = __reduce_add_sync(FULL, wide);  // 16-bit halves: at most m <= 16384 each
+                wide2 = __reduce_add_sync(FULL, wide2);
+                g[e][0] = wide & 0xffffu;
+                g[e][1] = wide >> 16;
+                g[e][2] = wide2 & 0xffffu;
+                g[e][3] = wide2 >> 16;
+            }
+            // the root's children in the reference's order, one per lane 0..3: (x low, y low), (high, low),
+            // (low, high), (high, high)
+            const bool xh = lane & 1, yh = lane & 2;
+            const uint32_t c0 = yh ? (xh ? g[2][2] : g[2][0]) : (xh ? g[0][2] : g[0][0]);
+            const uint32_t c1 = yh ? (xh ? g[2][3] : g[2][1]) : (xh ? g[0][3] : g[0][1]);
+            const uint32_t c2 = yh ? (xh ? g[3][2] : g[3][0]) : (xh ? g[1][2] : g[1][0]);
+            const uint32_t c3 = yh ? (xh ? g[3][3] : g[3][1]) : (xh ? g[1][3] : g[1][1]);
+            const uint32_t cc = c0 + c1 + c2 + c3;
+            const uint32_t area = (uint32_t)(xh ? nx_hi : nx_lo) *
+                                  (uint32_t)(yh ? bpos[4] - bpos[2] : bpos[2] - bpos[0]);
+            const bool wide_enough = 1 < (xh ? m - half : half) || 1 < (yh ? m - half : half);
+            const bool splittable = lane < 4 && wide_enough && cc > 2;
+            const bool leaf_now = lane < 4 && !splittable && cc > 0;
+            const unsigned msplit = __ballot_sync(FULL, splittable), mleaf = __ballot_sync(FULL, leaf_now);
+            const unsigned magain = __ballot_sync(FULL, splittable && chi_square_above(c0, c1, c2, c3, cc));
+            // leaves of the root's own step first, then the children from the last to the first
+            const int at = leaf_now ? __popc(mleaf & ((1u << lane) - 1u)) : __popc(mleaf) + __popc(msplit >> (lane + 1));
+            if (leaf_now || (splittable && !magain)) {
+                lnxy[nq + at] = cc;
+                lnxny[nq + at] = area;
+            }
+            nq += __popc(mleaf) + (magain ? 0 : __popc(msplit));
+            if (lane == slot) end = nq;
+            if (!magain) {
+                ++slot;
+                if (nq >= 32) flush();
+                continue;
+            }
+#pragma unroll 4
+            for (int k = lane; k < m; k += 32) xg[k] = xr[oY[k]] & 0x3fffu;
+            __syncwarp();
+            bool broken = false;
+            int64_t guard = 0;
+#pragma unroll 1
+            for (int c = 3; c >= 0; --c) {
+                if (!((msplit >> c) & 1u)) continue;
+                const uint32_t ccc = __shfl_sync(FULL, cc, c), ar = __shfl_sync(FULL, area, c);
+                if (!((magain >> c) & 1u)) {
+                    if (lane == 0) {
+                        lnxy[nq] = ccc;
+                        lnxny[nq] = ar;
+                    }
+                    ++nq;
+                    if (lane == slot) end = nq;
+                    continue;
+                }
+                if (lane == 0)
+                    stack[0] = ApWin{(uint16_t)((c & 1) ? half : 0), (uint16_t)((c >> 1) ? half : 0),
+                                     (uint16_t)((c & 1) ? m : half), (uint16_t)((c >> 1) ? m : half), ccc};
                 __syncwarp();
+                int top = 1;
+                bool from_grid = true;
+#pragma unroll 1
+                while (top > 0) {
+                    if (++guard > 16ll * m + 64) {  // cannot happen: every pushed window is smaller than its parent
+                        broken = true;
+                        break;
+                    }
+                    if (nq >= 32) flush();
+                    const ApWin wv = stack[top - 1];
+                    __syncwarp();
+                    const int mx = (wv.x1 + wv.x2) >> 1, my = (wv.y1 + wv.y2) >> 1;
+                    uint32_t d0, d1, d2, d3;
+                    if (from_grid) {  // the child itself: its counts and its split are known
+                        d0 = __shfl_sync(FULL, c0, c);
+                        d1 = __shfl_sync(FULL, c1, c);
+                        d2 = __shfl_sync(FULL, c2, c);
+                        d3 = __shfl_sync(FULL, c3, c);
+                    } else {
+                        const unsigned wl = mx - wv.x1, wa = wv.x2 - wv.x1;
+                        const int b1 = cY[my];
+                        // per y half: samples left of mx, and in the window
+                        auto scan = [&](int from, int to, uint32_t& low, uint32_t& high) {
+                            uint32_t l = 0, all = 0;
+#pragma unroll 2
+                            for (int k = from + lane; k < to; k += 32) {
+                                const unsigned x = (unsigned)xg[k] - wv.x1;
+                                l += x < wl;
+                                all += x < wa;
+                            }
+                            low = __reduce_add_sync(FULL, l);
+                            high = __reduce_add_sync(FULL, all) - low;
+                        };
+                        scan(cY[wv.y1], b1, d0, d1);
+                        scan(b1, cY[wv.y2], d2, d3);
+                    }
+                    --top;
+                    if (from_grid || chi_square_above(d0, d1, d2, d3, wv.npts)) {
+                        from_grid = false;
+                        const int sx1[4] = {wv.x1, mx, wv.x1, mx}, sx2[4] = {mx, wv.x2, mx, wv.x2};
+                        const int sy1[4] = {wv.y1, wv.y1, my, my}, sy2[4] = {my, my, wv.y2, wv.y2};
+                        const uint32_t sc[4] = {d0, d1, d2, d3};
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const bool split = ((sx1[u] + 1) < sx2[u] || (sy1[u] + 1) < sy2[u]) && sc[u] > 2;
+                            if (split) {
+                                if (top >= AP_STACK) {
+                                    broken = true;
+                                    continue;
+                                }
+                                if (lane == 0)
+                                    stack[top] = ApWin{(uint16_t)sx1[u], (uint16_t)sy1[u], (uint16_t)sx2[u],
+                                                       (uint16_t)sy2[u], sc[u]};
+                                ++top;
+                            } else if (sc[u] > 0) {
+                                if (lane == 0) {
+                                    lnxy[nq] = sc[u];
+                                    lnxny[nq] = (uint32_t)(cX[sx2[u]] - cX[sx1[u]]) * (uint32_t)(cY[sy2[u]] - cY[sy1[u]]);
+                                }
+                                ++nq;
+                            }
+                        }
+                    } else {
+                        if (lane == 0) {
+                            lnxy[nq] = wv.npts;
+                            lnxny[nq] = (uint32_t)(cX[wv.x2] - cX[wv.x1]) * (uint32_t)(cY[wv.y2] - cY[wv.y1]);
+                        }
+                        ++nq;
+                    }
+                    if (lane == slot) end = nq;
+                    __syncwarp();
+                    if (broken) break;
+                }
                 if (broken) break;
             }
-            ap_flush(lnxy, lnxny, nleaf, mi, lane);
-            if (lane == 0) {
-                float v = (float)(mi / (double)m + logm);
-                if (broken) {
-                    v = __int_as_float(0x7fc00000);
-                    atomicOr(a.flag, 2);
-                }
-                a.MI[(int64_t)i * a.ldmi + j] = v;
-                a.MI[(int64_t)j * a.ldmi + i] = v;
-            }
+            if (broken && lane == slot) broken_mine = true;
             __syncwarp();
+            ++slot;
+            if (nq >= 32) flush();
         }
         __syncthreads();
     }
@@ -376,7 +512,8 @@ cudaError_t launch_ap_mi(const uint16_t* xr, const uint16_t* order, const uint16
     a.ldmi = ldmi;
     a.next_i = next_i;
     a.flag = flag;
-    a.warp_bytes = (int)(AP_STACK * sizeof(ApWin) + 2 * AP_LEAVES * sizeof(uint32_t) + ((int64_t)m * 2 + 15) / 16 * 16);
+    a.warp_bytes = (int)(AP_STACK * sizeof(ApWin) + AP_LEAVES * (sizeof(double) + 2 * sizeof(uint32_t)) +
+                         ((int64_t)m * 2 + 15) / 16 * 16);
     int dev = 0, sms = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

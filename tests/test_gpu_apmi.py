@@ -96,3 +96,20 @@ def test_ap_mi_4096_genes(gpu, port):
     idx = np.random.default_rng(1).choice(n, 48, replace=False)
     R = port.ap_ranks(X[idx])
     assert_ap_close(A[np.ix_(idx, idx)], port.ap_mi(R))
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 7, 8, 31, 130, 1027, 16384])
+def test_ap_mi_small_sizes_and_large_tie_groups(gpu, port, m):
+    """Sample counts around the grid's boundaries, more pairs than a batch of 32, and genes whose samples
+    mostly share one rank (a quartile band then holds nearly all of them)."""
+    rng = np.random.default_rng(m)
+    n = 70 if m < 2000 else 5
+    X = rng.random((n, m)).astype(np.float32)
+    X[1] = 0.5
+    X[2] = np.where(rng.random(m) < 0.9, 0.25, X[2])
+    X[3] = np.round(X[3] * 2) / 2
+    X[4] = X[2]
+    R = port.ap_ranks(X)
+    # so few distinct terms that one log2 rounded the other way (log2 3 in an exact zero at m = 3) moves many
+    # entries by an ulp: the distance only, not the share of equal entries
+    assert_ap_close(gpu.ap_mi_ranks(R), port.ap_mi(R), exact_frac=0.0)
