@@ -47,8 +47,11 @@ constexpr int SC_ITEMS = 4;
 constexpr int SC_TILE = SC_THREADS * SC_ITEMS;
 constexpr int RS_THREADS = 256;                      // radix sort
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
+// Keys per thread: 16, or 4 where tiles of 4,096 keys would leave most SMs without one (a block ranks its
+// rows one after the other; 42,000 keys: 26 -> 11 us a pass without its scan).
+constexpr int RS_ITEMS = 16, RS_ITEMS_FEW = 4;
+constexpr int64_t RS_FEW = 152 * RS_THREADS * RS_ITEMS;
+constexpr int rs_items(int64_t n) { return n <= RS_FEW ? RS_ITEMS_FEW : RS_ITEMS; }
 // Directory width and CTAs per SM: 20 bits (a 4 MB directory, L2-resident) and 4 CTAs
 // measured best of 16/18/20 bits x 3/4 CTAs on the evaluations of a 32,768-gene network.
 #ifndef MCPG_RC_DIR_BITS
@@ -222,9 +225,42 @@ __global__ void __launch_bounds__(SC_THREADS) scan_tile_down(const T* in, int64_
     }
 }
 
+// The whole scan in one block, a tile after the other (16 elements a thread instead of SC_ITEMS: slower,
+// 10.8 against 9.7 us for 10,496 elements: its accesses are 64 and 128 bytes apart).
+template <typename T>
+__global__ void __launch_bounds__(SC_THREADS) scan_few_tiles(const T* in, int64_t n, uint64_t* out) {
+    __shared__ uint64_t sw[32];
+    uint64_t carry = 0;
+    for (int64_t c0 = 0; c0 < n; c0 += SC_TILE) {
+        const int64_t base = c0 + (int64_t)threadIdx.x * SC_ITEMS;
+        uint64_t v[SC_ITEMS], s = 0;
+#pragma unroll
+        for (int k = 0; k < SC_ITEMS; ++k) {
+            v[k] = base + k < n ? (uint64_t)in[base + k] : 0;
+            s += v[k];
+        }
+        uint64_t total;
+        uint64_t run = carry + block_excl_scan(s, sw, total);
+#pragma unroll
+        for (int k = 0; k < SC_ITEMS; ++k) {
+            if (base + k < n) out[base + k] = run;
+            run += v[k];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
 template <typename T>
 cudaError_t scan_any(const T* in, int64_t n, uint64_t* out, uint64_t* tmp, cudaStream_t st, int64_t* launches) {
     if (n <= 0) return cudaMemsetAsync(out, 0, sizeof(uint64_t), st);
+    // One launch (about 3 us a tile) instead of three of about 3 us each and the gaps between them: the block
+    // histograms of a radix pass over up to 98,304 keys.
+    if (n <= 6 * SC_TILE) {
+        scan_few_tiles<T><<<1, SC_THREADS, 0, st>>>(in, n, out);
+        if (launches) ++*launches;
+        return cudaGetLastError();
+    }
     const int64_t nb = ceil_div(n, SC_TILE);
     scan_tile_sums<T><<<(unsigned)nb, SC_THREADS, 0, st>>>(in, n, tmp);
     scan_parts<<<1, SC_THREADS, 0, st>>>(tmp, nb, out + n);
@@ -300,14 +336,15 @@ __global__ void combo_keys_kernel(ComboSrc c, uint32_t* keys, int* nan_flag) {
 }
 
 // ---- LSD radix sort of 32-bit keys ----
+template <int ITEMS>
 __global__ void __launch_bounds__(RS_THREADS) radix_hist_kernel(const uint32_t* keys, int64_t n, int shift,
                                                                 uint32_t* bh, int64_t nblk) {
     __shared__ uint32_t h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * RS_TILE;
+    const int64_t base = (int64_t)blockIdx.x * (RS_THREADS * ITEMS);
 #pragma unroll 4
-    for (int k = 0; k < RS_ITEMS; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const int64_t i = base + k * RS_THREADS + threadIdx.x;
         if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
     }
@@ -316,10 +353,11 @@ __global__ void __launch_bounds__(RS_THREADS) radix_hist_kernel(const uint32_t* 
 }
 
 
-// Stable scatter: warp w owns tile elements [w*512, (w+1)*512) read as 16 rows
+// Stable scatter: warp w owns tile elements [w*32*ITEMS, (w+1)*32*ITEMS) read as ITEMS rows
 // of 32 lanes; equal digits are ranked in (row, lane) order with
 // __match_any_sync, then offset by the same digit in earlier warps of the block
 // and in earlier blocks (the digit-major scanned histogram).
+template <int ITEMS>
 __global__ void __launch_bounds__(RS_THREADS) radix_scatter_kernel(const uint32_t* in, uint32_t* out, int64_t n,
                                                                    int shift, const uint64_t* off, int64_t nblk) {
     __shared__ uint32_t wc[RS_WARPS][256];
@@ -328,11 +366,11 @@ __global__ void __launch_bounds__(RS_THREADS) radix_scatter_kernel(const uint32_
     for (int d = threadIdx.x; d < RS_WARPS * 256; d += RS_THREADS) (&wc[0][0])[d] = 0;
     boff[threadIdx.x] = off[(int64_t)threadIdx.x * nblk + blockIdx.x];
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * RS_TILE + (int64_t)w * (RS_ITEMS * 32);
-    uint32_t key[RS_ITEMS], rank[RS_ITEMS];
+    const int64_t base = ((int64_t)blockIdx.x * RS_WARPS + w) * (ITEMS * 32);
+    uint32_t key[ITEMS], rank[ITEMS];
     const uint32_t lt = lanemask_lt();
 #pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const int64_t i = base + k * 32 + lane;
         const bool valid = i < n;
         key[k] = valid ? in[i] : 0u;
@@ -360,7 +398,7 @@ __global__ void __launch_bounds__(RS_THREADS) radix_scatter_kernel(const uint32_
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const int64_t i = base + k * 32 + lane;
         if (i < n) {
             const uint32_t d = (key[k] >> shift) & 255u;
@@ -631,7 +669,8 @@ __global__ void __launch_bounds__(CV_THREADS) curve_kernel(const uint32_t* X, in
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nX; k += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t x = X[k];
         if (k > 0 && X[k - 1] == x) continue;  // not the first of an equal run
-        int64_t lo = k + 1, hi = nX;          // end of the run
+        int64_t lo = k + 1, hi = nX;          // end of the run: mostly the next key already
+        if (lo < nX && X[lo] != x) hi = lo;
         while (lo < hi) {
             const int64_t mid = (lo + hi) >> 1;
             if (X[mid] == x) lo = mid + 1; else hi = mid;
@@ -671,13 +710,35 @@ __global__ void __launch_bounds__(CV_THREADS) curve_kernel(const uint32_t* X, in
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        Neu p, r;
-        for (unsigned i = 0; i < gridDim.x; ++i) {
+    if (!last) return;
+    // The last block merges the blocks' sums: a thread a strided share, then warps and block as above.  (One
+    // thread merging 256 blocks, a chain of dependent FP64 additions each, took 130 of the kernel's 177 us.)
+    __threadfence();
+    Neu p, r;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += CV_THREADS) {
+        Neu a, b;
+        a.s = __ldcg(part + 4 * i); a.c = __ldcg(part + 4 * i + 1);
+        b.s = __ldcg(part + 4 * i + 2); b.c = __ldcg(part + 4 * i + 3);
+        p.merge(a);
+        r.merge(b);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        Neu a, b;
+        a.s = __shfl_down_sync(FULL, p.s, o);
+        a.c = __shfl_down_sync(FULL, p.c, o);
+        b.s = __shfl_down_sync(FULL, r.s, o);
+        b.c = __shfl_down_sync(FULL, r.c, o);
+        p.merge(a);
+        r.merge(b);
+    }
+    if (lane == 0) {
+        sh[w][0] = p.s; sh[w][1] = p.c; sh[w][2] = r.s; sh[w][3] = r.c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < CV_THREADS / 32; ++i) {
             Neu a, b;
-            a.s = __ldcg(part + 4 * i); a.c = __ldcg(part + 4 * i + 1);
-            b.s = __ldcg(part + 4 * i + 2); b.c = __ldcg(part + 4 * i + 3);
+            a.s = sh[i][0]; a.c = sh[i][1]; b.s = sh[i][2]; b.c = sh[i][3];
             p.merge(a);
             r.merge(b);
         }
@@ -700,7 +761,7 @@ int64_t truth_items(const TruthRegion& r) {
     return r.rows * ceil_div(r.cols, EV_CHUNK);
 }
 int64_t scan_tmp_elems(int64_t n) { return ceil_div(n > 0 ? n : 1, SC_TILE); }
-int64_t radix_blocks(int64_t n) { return ceil_div(n > 0 ? n : 1, RS_TILE); }
+int64_t radix_blocks(int64_t n) { return ceil_div(n > 0 ? n : 1, RS_THREADS * rs_items(n)); }
 int64_t curve_part_elems() { return 4 * CV_MAX_BLOCKS; }
 int64_t rank_dir_elems() { return RC_DIR; }
 
@@ -766,14 +827,19 @@ cudaError_t launch_radix_sort(uint32_t* keys, uint32_t* alt, int64_t n, uint32_t
                               uint64_t* tmp, cudaStream_t st, int64_t* launches) {
     if (n <= 1) return cudaSuccess;
     const int64_t nblk = radix_blocks(n);
+    const bool few = rs_items(n) == RS_ITEMS_FEW;
     uint32_t* src = keys;
     uint32_t* dst = alt;
     for (int pass = 0; pass < 4; ++pass) {
         const int shift = 8 * pass;
-        radix_hist_kernel<<<(unsigned)nblk, RS_THREADS, 0, st>>>(src, n, shift, bh, nblk);
+        if (few) radix_hist_kernel<RS_ITEMS_FEW><<<(unsigned)nblk, RS_THREADS, 0, st>>>(src, n, shift, bh, nblk);
+        else radix_hist_kernel<RS_ITEMS><<<(unsigned)nblk, RS_THREADS, 0, st>>>(src, n, shift, bh, nblk);
         cudaError_t e = scan_any<uint32_t>(bh, 256 * nblk, bh_off, tmp, st, launches);
         if (e != cudaSuccess) return e;
-        radix_scatter_kernel<<<(unsigned)nblk, RS_THREADS, 0, st>>>(src, dst, n, shift, bh_off, nblk);
+        if (few)
+            radix_scatter_kernel<RS_ITEMS_FEW><<<(unsigned)nblk, RS_THREADS, 0, st>>>(src, dst, n, shift, bh_off, nblk);
+        else
+            radix_scatter_kernel<RS_ITEMS><<<(unsigned)nblk, RS_THREADS, 0, st>>>(src, dst, n, shift, bh_off, nblk);
         if (launches) *launches += 2;
         uint32_t* t = src;
         src = dst;
@@ -788,7 +854,8 @@ static cudaError_t rank_prep(const uint32_t* X, int64_t nX, uint64_t* lt, uint64
     cudaError_t e = cudaMemsetAsync(lt, 0, (size_t)(nX + 1) * sizeof(uint64_t), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(eq, 0, (size_t)(nX + 1) * sizeof(uint64_t), st);
     if (e != cudaSuccess) return e;
-    rank_dir_kernel<<<grid_for(RC_DIR, 256, 152 * 2), 256, 0, st>>>(X, nX, dir);
+    // (one entry per thread: a search is a chain of dependent loads)
+    rank_dir_kernel<<<grid_for(RC_DIR, 256, 1 << 13), 256, 0, st>>>(X, nX, dir);
     if (launches) ++*launches;
     return cudaGetLastError();
 }
