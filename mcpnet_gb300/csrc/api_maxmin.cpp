@@ -293,7 +293,8 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
             CK(h, mcpg::launch_ranked_order(q.L, n, q.rank, q.perm, h->stream, &h->launches), "order kernel");
             CK(h, mcpg::launch_ranked_transpose(a, la, n, n, 1, q.perm, rk.XT, r.ldt, rk.cnt, h->stream, &h->launches),
                "transpose kernel");
-            CK(h, mcpg::launch_ranked_dpi(r, q.rank, p.tol_mult, out, ldo, mask, n, gone, h->stream, &h->launches),
+            CK(h, mcpg::launch_ranked_dpi(r, q.rank, p.tol_mult, out, ldo, mask, n, gone, gone + 1, h->stream,
+                                          &h->launches),
                "ranked DPI kernels");
         }
         unsigned long long got[3] = {0, 0, 0};  // NaN seen, pending, removed

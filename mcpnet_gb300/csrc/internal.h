@@ -105,10 +105,10 @@ cudaError_t launch_ranked_transpose(const float* X, int64_t ldx, int64_t rows, i
 // symmetric: O == X, owners in the order of perm, only columns at or after the owner.
 cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t st, int64_t* launches);
 // The DPI filter of O == X (lists and XT with skip_diag): out / mask in gene order, *removed += the
-// entries that changed; nothing when the ranked form gave up.
+// entries that changed; nothing when the ranked form gave up.  removed, asym: zeroed before.
 cudaError_t launch_ranked_dpi(const RankedArgs& a, const int* rank, double tol_mult, float* out, int64_t ldo,
-                              uint8_t* mask, int64_t ldmask, unsigned long long* removed, cudaStream_t st,
-                              int64_t* launches);
+                              uint8_t* mask, int64_t ldmask, unsigned long long* removed, unsigned long long* asym,
+                              cudaStream_t st, int64_t* launches);
 // C and the first k attaining it (as MM_WITNESS) after launch_ranked_walk; PK: as P, open_n: a zeroed count
 // (above pending_cap: gave up, and nothing is written).
 cudaError_t launch_ranked_witness(const RankedArgs& a, int symmetric, const int* rank, int* PK,

@@ -30,8 +30,9 @@
 // host synchronisation: the sequence can be captured and stays asynchronous.
 //
 // Measured on MI-like matrices (symmetric product with ratio, whole call; exhaustive form ->
-// this one): 20,000 genes 338 -> 19.7 ms (walk 13.5, lists 2.9, finish 1.9, transpose 1.1 ms);
-// M1..M3 with ratios at 2,000 genes 1.79 -> 0.48 ms; 300 genes, one product, 71 -> 66 us.
+// this one): 20,000 genes 338 -> 18.8 ms (walk 13.5, lists 2.1, finish 1.6, transpose 1.1 ms); M1..M3
+// with ratios at 2,000 genes 1.79 -> 0.46 ms; 300 genes, one product, 71 -> 49 us.  ncu at 8,192 genes: the
+// walk reads 18.9 TB/s from L2, 79 % of what the L1s take in.
 #include <float.h>
 #include <math.h>
 
@@ -168,18 +169,43 @@ __global__ void __launch_bounds__(LIST_TPB) lists_kernel(const float* __restrict
     while (p2 < count) p2 <<= 1;
     for (int t = count + tid; t < p2; t += LIST_TPB) buf[t] = 0;
     __syncthreads();
-    for (int s = 2; s <= p2; s <<= 1)
-        for (int j = s >> 1; j > 0; j >>= 1) {
-            for (int t = tid; t < p2 / 2; t += LIST_TPB) {
-                const int x = ((t & ~(j - 1)) << 1) | (t & (j - 1)), y = x | j;
-                const unsigned long long a = buf[x], b = buf[y];
-                if ((a < b) == ((x & s) == 0)) {
-                    buf[x] = b;
-                    buf[y] = a;
+    if (p2 == LIST_TPB) {
+        // one entry per thread: partners less than a warp apart exchange by shuffle, without a barrier (shorter
+        // lists leave warps idle here and sort faster below: 44 against 54 us for 2,000 rows)
+        unsigned long long v = buf[tid];
+        for (int s = 2; s <= LIST_TPB; s <<= 1) {
+            const bool down = (tid & s) == 0;
+            for (int j = s >> 1; j > 0; j >>= 1) {
+                unsigned long long u;
+                if (j >= 32) {
+                    __syncthreads();
+                    buf[tid] = v;
+                    __syncthreads();
+                    u = buf[tid ^ j];
+                } else {
+                    u = __shfl_xor_sync(FULL, v, j);
                 }
+                const bool first = (tid & j) == 0;  // the lower position keeps the larger where descending
+                v = (first == down) ? (u > v ? u : v) : (u < v ? u : v);
             }
-            __syncthreads();
         }
+        __syncthreads();
+        buf[tid] = v;
+        __syncthreads();
+    } else {
+        for (int s = 2; s <= p2; s <<= 1)
+            for (int j = s >> 1; j > 0; j >>= 1) {
+                for (int t = tid; t < p2 / 2; t += LIST_TPB) {
+                    const int x = ((t & ~(j - 1)) << 1) | (t & (j - 1)), y = x | j;
+                    const unsigned long long a = buf[x], b = buf[y];
+                    if ((a < b) == ((x & s) == 0)) {
+                        buf[x] = b;
+                        buf[y] = a;
+                    }
+                }
+                __syncthreads();
+            }
+    }
     const int padded = (count + BATCH - 1) / BATCH * BATCH;
     uint2* out = L.entries + (int64_t)i * L.pitch;
     for (int t = tid; t < padded; t += LIST_TPB) {
@@ -413,10 +439,23 @@ __global__ void __launch_bounds__(512) finish_kernel(const RankedArgs a, const i
                 *reinterpret_cast<float4*>(prow + j) = *reinterpret_cast<const float4*>(src + j);
             __syncthreads();
         }
-        for (int j = threadIdx.x; j < cols; j += 512) {
-            const float v = GATHER ? prow[crank[j]] : src[j];
-            if (C) C[i * ldc + j] = v;
-            if (R) R[i * ldr + j] = ratio_value(E[i * lde + j], v);
+        for (int j0 = threadIdx.x; j0 < cols; j0 += 4 * 512) {  // four columns' loads in flight
+            int c[4];
+            float e[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = j0 + u * 512;
+                c[u] = GATHER && j < cols ? crank[j] : j;
+                e[u] = R && j < cols ? E[i * lde + j] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = j0 + u * 512;
+                if (j >= cols) break;
+                const float v = GATHER ? prow[c[u]] : src[j];
+                if (C) C[i * ldc + j] = v;
+                if (R) R[i * ldr + j] = ratio_value(e[u], v);
+            }
         }
     }
 }
@@ -581,14 +620,64 @@ __global__ void __launch_bounds__(256) witness_finish_kernel(const RankedArgs a,
 // output settled as soon as its maximum reaches the threshold or no later entry can.  On MI
 // matrices nearly every pair is decided by its first few entries.  P receives a value
 // on the right side of both orientations' thresholds.  Measured (whole call, tolerance 0.1; the tiled
-// first-phase form -> this one): 20,000 genes 69.4 -> 14.8 ms (walk 8.3, lists 2.7, finish 2.4 ms), 2,000
-// genes 355 -> 188 us, 256 genes 227 -> 62 us.
-__device__ __forceinline__ float dpi_threshold(float e, double tm) { return (float)((double)e * tm); }
+// first-phase form -> this one): 20,000 genes 69.4 -> 11.3 ms (walk 6.4, lists 2.1, finish 1.2 ms; 14.8 ms
+// with the thresholds' products in FP64 and gathered for both orientations), 2,000 genes 355 -> 174 us.
+// The threshold (float)(e * tm) with the product in double, mostly without the FP64 pipe (16 clocks of an SM
+// per warp instruction): e times tm as a pair of floats, exact to 2^-45.  Where the rounding to float is
+// that far from a tie, it is the reference's; else, and outside the range the pair is good for, the double
+// product runs.
+struct DpiMult {
+    double tm;
+    float hi, lo;
+    bool pair;
+};
+DpiMult dpi_mult(double tm) {
+    DpiMult m;
+    m.tm = tm;
+    m.hi = (float)tm;
+    m.pair = isfinite(m.hi);
+    m.lo = m.pair ? (float)(tm - (double)m.hi) : 0.0f;
+    return m;
+}
+__device__ __forceinline__ float dpi_threshold(float e, const DpiMult& m) {
+    if (m.pair) {
+        const float ph = __fmul_rn(e, m.hi);
+        const float lo = __fmaf_rn(e, m.lo, __fmaf_rn(e, m.hi, -ph));
+        const float r = __fadd_rn(ph, lo);
+        const float err = __fadd_rn(__fsub_rn(ph, r), lo);
+        const uint32_t u = __float_as_uint(r) & 0x7fffffffu;
+        const float ulp = __uint_as_float(((u >> 23) - 23u) << 23);
+        if (u > 0x0d000000u && u < 0x7e000000u && (u & 0x7fffffu) && fabsf(err) < __fmul_rn(0.4999f, ulp)) return r;
+        if (e == 0.0f) return ph;
+    }
+    return (float)((double)e * m.tm);
+}
 __device__ __forceinline__ bool dpi_open(float acc, float next, float t0, float t1) {
     return (acc < t0 && next >= t0) || (acc < t1 && next >= t1);
 }
 
-__global__ void __launch_bounds__(OWN * 32) dpi_walk_kernel(const RankedArgs a, double tm) {
+// *asym = 1 when some A[i][j] != A[j][i] (64 x 64 tiles on and above the diagonal).
+__global__ void __launch_bounds__(256) symmetry_kernel(const float* __restrict__ A, int64_t lda, int n,
+                                                       unsigned long long* asym) {
+    __shared__ float tile[64][65];
+    const int bi = blockIdx.y * 64, bj = blockIdx.x * 64;
+    if (bj < bi || *(volatile unsigned long long*)asym) return;
+    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+#pragma unroll
+    for (int r = ty; r < 64; r += 4)
+        tile[r][tx] = bi + r < n && bj + tx < n ? A[(int64_t)(bi + r) * lda + bj + tx] : 0.0f;
+    __syncthreads();
+    bool differ = false;
+#pragma unroll
+    for (int r = ty; r < 64; r += 4) {
+        const float v = bj + r < n && bi + tx < n ? A[(int64_t)(bj + r) * lda + bi + tx] : 0.0f;
+        differ |= v != tile[tx][r];
+    }
+    if (differ) *asym = 1;
+}
+
+__global__ void __launch_bounds__(OWN * 32) dpi_walk_kernel(const RankedArgs a, const DpiMult tm,
+                                                           const unsigned long long* asym) {
     __shared__ float tile[OWN][COLS + 4];
     if (__syncthreads_or(threadIdx.x == 0 && gave_up(a))) return;
     const int o0 = blockIdx.x * OWN, p0 = blockIdx.y * COLS;
@@ -603,14 +692,15 @@ __global__ void __launch_bounds__(OWN * 32) dpi_walk_kernel(const RankedArgs a, 
         const float* col = a.XT + p;
         float acc[4], t0[4], t1[4];
         {
+            const bool symmetric = asym && *asym == 0;  // A[x][z] is A[z][x] then: no gather through the order
             const float4 e1 = ldg4(col + (int64_t)i * a.ldt);  // A[z][x]
             const float v1[4] = {e1.x, e1.y, e1.z, e1.w};
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const bool live = p + c > o && p + c < a.cols;  // z == x goes in any case
                 acc[c] = -INFINITY;
-                t0[c] = live ? dpi_threshold(__ldg(a.O + (int64_t)i * a.ldo + a.perm[p + c]), tm) : -INFINITY;
                 t1[c] = live ? dpi_threshold(v1[c], tm) : -INFINITY;
+                t0[c] = !live || symmetric ? t1[c] : dpi_threshold(__ldg(a.O + (int64_t)i * a.ldo + a.perm[p + c]), tm);
             }
         }
         auto any_open = [&](float next) {
@@ -684,7 +774,7 @@ __global__ void __launch_bounds__(OWN * 32) dpi_walk_kernel(const RankedArgs a, 
 }
 
 // One warp per pending pair: the other row's list, then both whole rows without x and z.
-__global__ void __launch_bounds__(256) dpi_ranked_pending_kernel(const RankedArgs a, double tm) {
+__global__ void __launch_bounds__(256) dpi_ranked_pending_kernel(const RankedArgs a, const DpiMult tm) {
     if (gave_up(a)) return;
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -729,7 +819,7 @@ __global__ void __launch_bounds__(256) dpi_ranked_pending_kernel(const RankedArg
 }
 
 // out = the entries that stay, mask, and the number of entries that changed.
-__global__ void __launch_bounds__(512) dpi_finish_kernel(const RankedArgs a, const int* __restrict__ rank, double tm,
+__global__ void __launch_bounds__(512) dpi_finish_kernel(const RankedArgs a, const int* __restrict__ rank, const DpiMult tm,
                                                          float* __restrict__ out, int64_t ldo, uint8_t* __restrict__ mask,
                                                          int64_t ldmask, unsigned long long* removed) {
     extern __shared__ float prow[];
@@ -743,13 +833,25 @@ __global__ void __launch_bounds__(512) dpi_finish_kernel(const RankedArgs a, con
         for (int j = threadIdx.x * 4; j < n; j += 512 * 4)
             *reinterpret_cast<float4*>(prow + j) = *reinterpret_cast<const float4*>(src + j);
         __syncthreads();
-        for (int j = threadIdx.x; j < n; j += 512) {
-            const float e = row[j];
-            const bool del = i == j || prow[rank[j]] >= dpi_threshold(e, tm);
-            const float o = del ? 0.0f : e;
-            out[i * ldo + j] = o;
-            cnt += (o != e);
-            if (mask) mask[i * ldmask + j] = del ? 1 : 0;
+        for (int j0 = threadIdx.x; j0 < n; j0 += 4 * 512) {  // four columns' loads in flight
+            int c[4];
+            float e[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = j0 + u * 512;
+                c[u] = j < n ? rank[j] : 0;
+                e[u] = j < n ? row[j] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = j0 + u * 512;
+                if (j >= n) break;
+                const bool del = i == j || prow[c[u]] >= dpi_threshold(e[u], tm);
+                const float o = del ? 0.0f : e[u];
+                out[i * ldo + j] = o;
+                cnt += (o != e[u]);
+                if (mask) mask[i * ldmask + j] = del ? 1 : 0;
+            }
         }
     }
 #pragma unroll
@@ -764,6 +866,7 @@ int isqrt_ceil(int64_t v) { return (int)ceil(sqrt((double)v)); }
 int ranked_list_cap(int64_t k) {
     // four square roots of the candidate count cover 99 % of the outputs of the measured matrices
     int64_t c = (4 * (int64_t)isqrt_ceil(k) + 31) / 32 * 32;
+    if (c > LIST_TPB && c <= LIST_TPB + 128) c = LIST_TPB;  // one entry per thread of the sort (k up to 25,600)
     return (int)(c > LIST_MAX ? LIST_MAX : c);
 }
 
@@ -826,17 +929,22 @@ cudaError_t launch_ranked_finish(const RankedArgs& a, const int* rrank, const in
 }
 
 cudaError_t launch_ranked_dpi(const RankedArgs& a, const int* rank, double tol_mult, float* out, int64_t ldo,
-                              uint8_t* mask, int64_t ldmask, unsigned long long* removed, cudaStream_t st,
-                              int64_t* launches) {
-    if (launches) *launches += 3;
+                              uint8_t* mask, int64_t ldmask, unsigned long long* removed, unsigned long long* asym,
+                              cudaStream_t st, int64_t* launches) {
+    if (launches) *launches += 4;
     dim3 grid((unsigned)ceil_div(a.owners, OWN), (unsigned)ceil_div(a.cols, COLS));
-    dpi_walk_kernel<<<grid, OWN * 32, 0, st>>>(a, tol_mult);
-    dpi_ranked_pending_kernel<<<152 * 8, 256, 0, st>>>(a, tol_mult);
+    const DpiMult tm = dpi_mult(tol_mult);
+    // (a matrix that fits L2 gathers its thresholds cheaply: no check there)
+    if (a.owners < 4096) asym = nullptr;
+    const unsigned tiles = (unsigned)ceil_div(a.owners, 64);
+    if (asym) symmetry_kernel<<<dim3(tiles, tiles), 256, 0, st>>>(a.O, a.ldo, a.owners, asym);
+    dpi_walk_kernel<<<grid, OWN * 32, 0, st>>>(a, tm, asym);
+    dpi_ranked_pending_kernel<<<152 * 8, 256, 0, st>>>(a, tm);
     const size_t smem = (size_t)((a.cols + 3) / 4 * 4) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(dpi_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dpi_finish_kernel<<<(unsigned)(a.owners < 152 * 16 ? a.owners : 152 * 16), 512, smem, st>>>(
-        a, rank, tol_mult, out, ldo, mask, ldmask, removed);
+        a, rank, tm, out, ldo, mask, ldmask, removed);
     return cudaGetLastError();
 }
 

@@ -172,3 +172,30 @@ def test_witnesses_equal_the_first_attaining_candidate(gpu, kind, rows, cols, k)
             want = np.where(value == -np.inf, -1, first)
             assert np.array_equal(K[i], want), i
             assert np.array_equal(C[i], value), i
+
+
+def test_dpi_thresholds_at_rounding_ties(gpu, port):
+    """Entries over the float range, powers of two and their neighbours, where the product's rounding is
+    decided in its last bits; and a matrix large enough for the symmetry check."""
+    rng = np.random.default_rng(4)
+    n = 300
+    e = np.exp2(rng.integers(-40, 30, (n, n)).astype(np.float32)) * (1 + rng.integers(-3, 4, (n, n)) * np.float32(2.0 ** -23))
+    A = np.maximum(e, e.T).astype(np.float32)
+    for tol in (0.1, 0.2, 0.25, 0.5, 1.0 - 2.0 ** -20):
+        out, mask, removed = gpu.dpi(A, tol, want_mask=True)
+        oo, om, orem = port.dpi(A, tol)
+        assert np.array_equal(mask, om) and np.array_equal(bits(out), bits(oo)) and removed == orem
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_dpi_above_the_symmetry_check(gpu, port, symmetric):
+    rng = np.random.default_rng(8)
+    n = 4100
+    A = (rng.random((n, n), dtype=np.float32) ** 4) * np.exp(rng.standard_normal((n, 1))).astype(np.float32)
+    if symmetric:
+        A = np.maximum(A, A.T)
+    out, mask, _ = gpu.dpi(A, 0.1, want_mask=True)
+    rows = np.r_[0:20, 2000:2020, n - 20:n].astype(np.int64)
+    oo, om, _ = port.dpi_rows(A, rows, 0.1)
+    assert np.array_equal(mask[rows], om)
+    assert np.array_equal(bits(out[rows]), bits(oo))
