@@ -847,13 +847,21 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
                     for (int j = 0; j < SUB; ++j) {
                         const int64_t gs = g * SUB + j;  // slice slot sequence
                         if ((int)(gs % NPROD) != pid) continue;
+                        // A missing slice asks nothing of rank 1: the MMAs pass it on the leader's arrival
+                        // alone.  So rank 1 must not wait for its slot either: a thread that lags (its CTA's
+                        // epilogue storing to host memory, say) could find the slot's barrier a phase further,
+                        // with the awaited parity come round again, and wait for a commit that needs its own
+                        // next load.  The wait it skips is not needed by the slot's next use: the thread's last
+                        // real slice, at most 6 before, was seen to be free, so the phase before the awaited
+                        // one (14 slices back) is complete.
+                        if (j >= ns && !leader) continue;
                         const int r = (int)(gs % SLOTS);
                         const int64_t u = gs / SLOTS;
                         if (u > 0 && !(ok = mbar_wait_abortable(empty0 + 8 * r, (uint32_t)((u - 1) & 1), args.err,
                                                                 abort_flag, args.wait_ns)))
                             break;
                         if (j >= ns) {
-                            if (leader) mbar_arrive(full0 + 8 * s);
+                            mbar_arrive(full0 + 8 * s);
                             continue;
                         }
                         if (leader) mbar_expect_tx(full0 + 8 * s, 2u * slice_tx);  // this slice of both CTAs

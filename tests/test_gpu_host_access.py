@@ -175,3 +175,16 @@ def test_host_entry_points_in_place(gpu, built_lib):
         a, b, bits = _both(gpu, fn)
         assert bits == want_bits, name
         _same(a, b)
+
+
+def test_tensor_core_mi_into_host_memory_never_times_out(gpu, built_lib):
+    """Epilogue stores to host memory slow one CTA of a pair now and then.  With 400 samples (7 slices in
+    stages of 3) its producers then lagged behind slices that only the leader announces, missed a phase of
+    the slot's barrier and the pair waited for itself: one call in 200 to 10,000 reported a timeout."""
+    X = {n: built_lib.synth_grn(n, 400, seed=n) for n in (1100, 1601, 2100)}
+    first = {n: gpu.bspline_mi(x, 10, 3, "bf16f8") for n, x in X.items()}
+    for _ in range(400):
+        for n, x in X.items():
+            A = gpu.bspline_mi(x, 10, 3, "bf16f8")
+            assert np.array_equal(A, first[n])
+            gpu.dpi(A, 0.1, want_mask=True)
