@@ -95,6 +95,7 @@ enum Slot {
     S_RK_P,      // ranked max-min: the product in strength order
     S_RK_L0,     // ranked max-min: candidate lists of the first operand
     S_RK_L1,     // ranked max-min: candidate lists of the second operand
+    S_RK_LX,     // ranked max-min: candidate lists of a product's other operand
     S_RK_PEND,   // ranked max-min: pending outputs
     S_RK_CNT,    // ranked max-min: counters
     S_RK_K,      // ranked max-min: witnesses in strength order

@@ -31,9 +31,9 @@ struct Ranked {
     int64_t cap = 0;
     unsigned long long* cnt = nullptr;  // [0]: NaN seen, [1..]: a pending count per product
     int used = 1;
-    RankedSet set[2];
+    RankedSet set[2], other;
 };
-constexpr int RANKED_COUNTERS = 8;
+constexpr int RANKED_COUNTERS = 16;
 
 // Decides whether this call's products (at most rows x cols over k) take the ranked form, and lays out
 // its scratch.  Dense below
@@ -45,7 +45,7 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
     if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || rows < 8 || k > 32768 || rows > 50000 || cols > 50000) return;
     const int64_t most = std::max(rows, cols), lx = round_up(most, 128);  // either operand may own the lists
     const int64_t pitch = mcpg::ranked_list_cap(k);
-    r.cap = std::max<int64_t>(4096, rows * cols / 64);
+    r.cap = std::max<int64_t>(4096, rows * cols / 4);
     const size_t lbytes = (size_t)most * (size_t)pitch * sizeof(uint2) + (size_t)most * 5 * sizeof(int);
     struct { int slot; size_t bytes; void* p; } need[] = {
         {S_RK_CNT, RANKED_COUNTERS * sizeof(unsigned long long), nullptr},
@@ -54,6 +54,7 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
         {S_RK_PEND, (size_t)r.cap * sizeof(mcpg::RankedPending), nullptr},
         {S_RK_L0, lbytes, nullptr},
         {S_RK_L1, lists > 1 ? lbytes : 0, nullptr},
+        {S_RK_LX, lbytes, nullptr},
         {S_RK_K, witness ? (size_t)rows * (size_t)round_up(cols, 128) * sizeof(int) : 0, nullptr},
     };
     bool grow = false;
@@ -71,9 +72,10 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
     r.XT = (float*)need[1].p;
     r.P = (float*)need[2].p;
     r.pending = (mcpg::RankedPending*)need[3].p;
-    r.PK = (int*)need[6].p;
-    for (int s = 0; s < lists; ++s) {
-        RankedSet& q = r.set[s];
+    r.PK = (int*)need[7].p;
+    for (int s = 0; s < 3; ++s) {
+        if (s == 1 && lists < 2) continue;
+        RankedSet& q = s == 2 ? r.other : r.set[s];
         char* p = (char*)need[4 + s].p;
         q.L.entries = (uint2*)p;
         q.L.pitch = pitch;
@@ -92,7 +94,7 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
 // set s; swap: p.B owns (its rows carry the lists), which suits an A whose rows have no
 // pronounced largest values.  Falls back to the exhaustive kernel on the device.
 int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p, int mode, bool symm, bool swap) {
-    if (!r.on || r.used >= RANKED_COUNTERS) {
+    if (!r.on || r.used + 3 > RANKED_COUNTERS) {
         PROF(h, mode == mcpg::MM_WITNESS ? "maxmin_witness" : "maxmin");
         CK(h, mcpg::launch_maxmin(p, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
         return MCPG_OK;
@@ -121,12 +123,22 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     a.ldp = round_up(swap ? a.owners : a.cols, 128);
     a.direct = symm || !swap;
     a.mirror = symm || swap;
-    a.pending = r.pending; a.pending_cap = r.cap;
+    // A pending output that its lists do not settle reads two whole rows; 1/64 of the outputs may, which costs
+    // less than the exhaustive product.  A product of two operands lets more outputs pend, since the other
+    // operand's lists settle most: the MI matrix of 20,000 genes times its own M1 leaves a twentieth.
+    const int64_t outputs = (int64_t)a.owners * a.cols;
+    a.pending = r.pending; a.pending_cap = std::min(r.cap, std::max<int64_t>(4096, outputs / (symm ? 64 : 4)));
+    if (!symm) {
+        a.full_n = r.cnt + r.used++;
+        a.full_cap = (unsigned long long)std::max<int64_t>(4096, outputs / 64);
+    }
+    a.LX = r.other.L; a.lx_above = (unsigned long long)(outputs / 256);
     a.pending_n = r.cnt + r.used++;
     a.nan = r.cnt;
     CK(h, mcpg::launch_ranked_walk(a, symm ? 1 : 0, h->stream, &h->launches), "ranked max-min kernel");
     mcpg::MaxminParams d = p;
     d.run_above = a.pending_n; d.run_cap = (unsigned long long)a.pending_cap; d.run_nan = a.nan;
+    d.run_above3 = a.full_n; d.run_cap3 = a.full_cap;
     if (mode == mcpg::MM_WITNESS) {
         unsigned long long* open_n = r.cnt + r.used++;
         d.run_above2 = open_n;
@@ -284,7 +296,7 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
         r.XT = rk.XT; r.ldt = round_up(n, 128);
         r.P = rk.P; r.ldp = round_up(n, 128);
         r.direct = r.mirror = 1;
-        r.pending = rk.pending; r.pending_cap = rk.cap;
+        r.pending = rk.pending; r.pending_cap = std::max<int64_t>(4096, n * n / 64);
         r.nan = rk.cnt; r.pending_n = rk.cnt + 1;
         unsigned long long* gone = rk.cnt + 2;
         {
@@ -300,7 +312,7 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
         unsigned long long got[3] = {0, 0, 0};  // NaN seen, pending, removed
         CK(h, cudaMemcpyAsync(got, rk.cnt, sizeof got, cudaMemcpyDeviceToHost, h->stream), "read counters");
         CK(h, cudaStreamSynchronize(h->stream), "stream synchronize");
-        if (got[0] == 0 && got[1] <= (unsigned long long)rk.cap) {
+        if (got[0] == 0 && got[1] <= (unsigned long long)r.pending_cap) {
             if (removed) *removed = (int64_t)got[2];
             return MCPG_OK;
         }

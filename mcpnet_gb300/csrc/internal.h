@@ -61,6 +61,7 @@ struct MaxminParams {
     const unsigned long long* run_above; unsigned long long run_cap;
     const unsigned long long* run_nan;
     const unsigned long long* run_above2;
+    const unsigned long long* run_above3; unsigned long long run_cap3;  // nullable: or *run_above3 exceeds run_cap3
 };
 
 // symmetric != 0: A == B (same rows), rows == cols; only tiles on or above the
@@ -86,17 +87,23 @@ struct RankedArgs {
     const float* XT; int64_t ldt; // its transpose in column order perm, ldt a multiple of 128
     int owners, cols, k;
     RankedLists L;                // of O, in natural row order
+    RankedLists LX;               // of X (entries nullable), built when more than lx_above outputs are pending
+    unsigned long long lx_above;
     const int* perm;              // column p is row perm[p] of X (nullable: p)
     float* P; int64_t ldp;        // direct: P[o][p], mirror: P[p][o]
     int direct, mirror;
     RankedPending* pending; int64_t pending_cap;
     unsigned long long* pending_n;  // appended outputs; above pending_cap: the ranked form gave up
     const unsigned long long* nan;  // nonzero: an operand holds a NaN, and it gave up too
+    unsigned long long* full_n;     // (nullable) pending outputs that no list settled; above full_cap: gave up too
+    unsigned long long full_cap;
 };
 int ranked_list_cap(int64_t k);
 // skip_diag: entry (i, i) is not listed / -inf in XT
+// only_above (device, nullable): nothing unless it exceeds `above`
 cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64_t k, int skip_diag, const RankedLists& L,
-                                unsigned long long* nan, cudaStream_t st, int64_t* launches);
+                                unsigned long long* nan, cudaStream_t st, int64_t* launches,
+                                const unsigned long long* only_above = nullptr, unsigned long long above = 0);
 cudaError_t launch_ranked_order(const RankedLists& L, int64_t n, int* rank, int* perm, cudaStream_t st,
                                 int64_t* launches);
 cudaError_t launch_ranked_transpose(const float* X, int64_t ldx, int64_t rows, int64_t k, int skip_diag,

@@ -116,7 +116,8 @@ __global__ void __launch_bounds__(THREADS, MCPG_MM_MINB) maxmin_kernel(const Max
 
     int64_t ti = blockIdx.y, tj = blockIdx.x;
     if (SYMM && tj < ti) return;
-    if (p.run_above && *p.run_above <= p.run_cap && *p.run_nan == 0 && (!p.run_above2 || *p.run_above2 <= p.run_cap))
+    if (p.run_above && *p.run_above <= p.run_cap && *p.run_nan == 0 && (!p.run_above2 || *p.run_above2 <= p.run_cap) &&
+        (!p.run_above3 || *p.run_above3 <= p.run_cap3))
         return;
     const int64_t i0 = ti * BM, j0 = tj * BN;
     const bool mirror = SYMM && (tj != ti);

@@ -59,7 +59,8 @@ __device__ __forceinline__ float okey_value(int k) { return __int_as_float(k ^ (
 // Whether the ranked form gave up: too many pending outputs, or a NaN operand (the exhaustive
 // kernel behind it runs on the same condition).
 __device__ __forceinline__ bool gave_up(const RankedArgs& a) {
-    return *(const volatile unsigned long long*)a.pending_n > (unsigned long long)a.pending_cap || *a.nan != 0;
+    return *(const volatile unsigned long long*)a.pending_n > (unsigned long long)a.pending_cap || *a.nan != 0 ||
+           (a.full_n && *(const volatile unsigned long long*)a.full_n > a.full_cap);
 }
 // 16 bytes through the read-only path; volatile keeps a batch's loads together and in front
 // of their uses.
@@ -76,8 +77,10 @@ __device__ __forceinline__ float4 ldg4(const float* p) {
 template <int EPT>
 __global__ void __launch_bounds__(LIST_TPB) lists_kernel(const float* __restrict__ O, int64_t ldo, int rows, int k,
                                                          int want, int cap, int strength_at, int skip_diag,
-                                                         RankedLists L,
-                                                         unsigned long long* any_nan) {
+                                                         RankedLists L, unsigned long long* any_nan,
+                                                         const unsigned long long* only_above,
+                                                         unsigned long long only_cap) {
+    if (only_above && *only_above <= only_cap) return;  // uniform: no barrier is passed yet
     __shared__ unsigned long long buf[LIST_MAX];
     __shared__ int wcount[LIST_TPB / 32];
     __shared__ int fill;
@@ -367,13 +370,14 @@ __global__ void __launch_bounds__(OWN * 32) walk_kernel(const RankedArgs a) {
     }
 }
 
-// One warp per pending output: the other row's list (SYM), then both whole rows.
+// One warp per pending output: the other row's list (SYM, or where it was built), then both whole rows.
 template <bool SYM>
 __global__ void __launch_bounds__(256) pending_kernel(const RankedArgs a) {
     if (gave_up(a)) return;
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t count = (int64_t)*a.pending_n;
+    const bool other = !SYM && a.LX.entries && count > (int64_t)a.lx_above;
     for (int64_t x = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < count; x += nw) {
         const RankedPending d = a.pending[x];
         const int i = SYM ? a.perm[d.o] : d.o, j = a.perm ? a.perm[d.p] : d.p;
@@ -382,10 +386,11 @@ __global__ void __launch_bounds__(256) pending_kernel(const RankedArgs a) {
         float acc = d.m;
         float bound = a.L.bound[i];
         bool open = true;
-        if (SYM) {
-            const uint2* list = a.L.entries + (int64_t)j * a.L.pitch;
-            const int c = a.L.count[j];
-            const float bj = a.L.bound[j];
+        if (SYM || other) {
+            const RankedLists& L = SYM ? a.L : a.LX;
+            const uint2* list = L.entries + (int64_t)j * L.pitch;
+            const int c = L.count[j];
+            const float bj = L.bound[j];
             for (int t = 0; t < c && open; t += 32) {
                 if (t + lane < c) {
                     const uint2 e = __ldg(list + t + lane);
@@ -396,6 +401,11 @@ __global__ void __launch_bounds__(256) pending_kernel(const RankedArgs a) {
             }
             bound = fminf(bound, bj);
             if (open) open = !__any_sync(FULL, okey(acc) >= okey(bound));
+        }
+        if (open && a.full_n) {  // both whole rows: only so many of these
+            unsigned long long seen = 0;
+            if (lane == 0) seen = atomicAdd(a.full_n, 1ull);
+            if (__shfl_sync(FULL, seen, 0) >= a.full_cap) return;
         }
         const int kb = okey(bound);
         for (int t = 0; t < a.k && open; t += 128) {
@@ -871,15 +881,16 @@ int ranked_list_cap(int64_t k) {
 }
 
 cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64_t k, int skip_diag, const RankedLists& L,
-                                unsigned long long* nan, cudaStream_t st, int64_t* launches) {
+                                unsigned long long* nan, cudaStream_t st, int64_t* launches,
+                                const unsigned long long* only_above, unsigned long long above) {
     const int cap = ranked_list_cap(k), want = cap * 3 / 4, at = 2 * isqrt_ceil(k);
     if (k > (int64_t)LIST_TPB * 64 || L.pitch < cap) return cudaErrorInvalidValue;
     if (launches) ++*launches;
     const unsigned g = (unsigned)rows;
-    if (k <= LIST_TPB * 4) lists_kernel<4><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan);
-    else if (k <= LIST_TPB * 16) lists_kernel<16><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan);
-    else if (k <= LIST_TPB * 40) lists_kernel<40><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan);
-    else lists_kernel<64><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan);
+    if (k <= LIST_TPB * 4) lists_kernel<4><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
+    else if (k <= LIST_TPB * 16) lists_kernel<16><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
+    else if (k <= LIST_TPB * 40) lists_kernel<40><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
+    else lists_kernel<64><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
     return cudaGetLastError();
 }
 
@@ -906,6 +917,14 @@ cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t 
     else walk_kernel<false><<<grid, OWN * 32, 0, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    if (!symmetric && a.LX.entries) {
+        // An owner with many large entries against a row without: only the other row's list settles
+        // that early.  Its lists are built when such pairs are many (their reading costs as much as one
+        // pending output in 256).
+        e = launch_ranked_lists(a.X, a.ldx, a.cols, a.k, 0, a.LX, const_cast<unsigned long long*>(a.nan), st, launches,
+                                a.pending_n, a.lx_above);
+        if (e != cudaSuccess) return e;
+    }
     const unsigned g = 152 * 8;
     if (symmetric) pending_kernel<true><<<g, 256, 0, st>>>(a);
     else pending_kernel<false><<<g, 256, 0, st>>>(a);
