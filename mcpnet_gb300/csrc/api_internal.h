@@ -150,6 +150,15 @@ inline int cuda_fail(mcpg_handle* h, cudaError_t e, const char* what) {
         cudaError_t _e = (expr);                            \
         if (_e != cudaSuccess) return cuda_fail(h, _e, what); \
     } while (0)
+// Whether the handle's stream is being captured into a graph (or cannot tell).
+inline bool capturing(mcpg_handle* h) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return cs != cudaStreamCaptureStatusNone;
+}
 // Grow-only scratch slot.
 inline int scratch(mcpg_handle* h, int slot, size_t bytes, void** out) {
     if (bytes == 0) bytes = 16;

@@ -39,10 +39,13 @@ constexpr int RANKED_COUNTERS = 16;
 // its scratch.  Dense below
 // MCPG_RANKED_MIN candidates or rows (the ranked form's six launches cost more than one small
 // product), above the list kernel's 32,768 candidates or the finishing kernel's row buffer, where
-// the scratch cannot be had, and in a stream capture that would have to allocate it.
+// the scratch cannot be had, and in a stream capture: a graph of the exhaustive form holds no
+// scratch of the handle, so it may be replayed after the scratch has grown, on another stream
+// or after the handle is gone.
 void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t k, int lists, bool witness = false) {
     r = Ranked{};
     if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || rows < 8 || k > 32768 || rows > 50000 || cols > 50000) return;
+    if (capturing(h)) return;
     const int64_t most = std::max(rows, cols), lx = round_up(most, 128);  // either operand may own the lists
     const int64_t pitch = mcpg::ranked_list_cap(k);
     r.cap = std::max<int64_t>(4096, rows * cols / 4);
@@ -57,15 +60,6 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
         {S_RK_LX, lbytes, nullptr},
         {S_RK_K, witness ? (size_t)rows * (size_t)round_up(cols, 128) * sizeof(int) : 0, nullptr},
     };
-    bool grow = false;
-    for (auto& q : need) grow |= q.bytes > h->cap[q.slot];
-    if (grow) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
-        if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return;
-        }
-    }
     for (auto& q : need)
         if (q.bytes && scratch(h, q.slot, q.bytes, &q.p) != MCPG_OK) return;
     r.cnt = (unsigned long long*)need[0].p;

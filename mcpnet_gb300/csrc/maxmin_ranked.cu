@@ -27,7 +27,7 @@
 // more outputs stay open than the pending list holds (data without such structure: many
 // ties, closures), or an operand holds a NaN, a device-side count tells the exhaustive kernel
 // (maxmin.cu), which is always enqueued behind and otherwise returns at once, to run.  No
-// host synchronisation: the sequence can be captured and stays asynchronous.
+// host synchronisation: the sequence stays asynchronous.
 //
 // Measured on MI-like matrices (symmetric product with ratio, whole call; exhaustive form ->
 // this one): 20,000 genes 338 -> 18.8 ms (walk 13.5, lists 2.1, finish 1.6, transpose 1.1 ms); M1..M3
