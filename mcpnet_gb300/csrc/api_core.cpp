@@ -55,6 +55,10 @@ int mcpg_destroy(mcpg_handle* h) {
     mcpg_profile(h, 0);
     for (cudaEvent_t e : h->slab_events) cudaEventDestroy(e);
     if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
+    if (h->rk_done) {
+        cudaEventSynchronize(h->rk_done);
+        cudaEventDestroy(h->rk_done);
+    }
     for (int i = 0; i < NSLOTS; ++i)
         if (h->buf[i]) cudaFree(h->buf[i]);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
@@ -70,6 +74,7 @@ int mcpg_set_stream(mcpg_handle* h, void* s) {
         cudaStreamSynchronize(h->stream);
         cudaStreamDestroy(h->stream);
     }
+    h->rk_wait = h->rk_done != nullptr;
     h->stream = (cudaStream_t)s;
     h->own_stream = false;
     return MCPG_OK;

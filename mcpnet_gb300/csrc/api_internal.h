@@ -125,6 +125,9 @@ struct mcpg_handle {
     int ats = -1;
     int host_access = MCPG_HOST_ACCESS_AUTO;
     int last_direct = 0;  // MCPG_HOST_DIRECT_* of the last host call that can use them
+    // the ordered max-min form's scratch: its last use, and whether the stream was set since
+    cudaEvent_t rk_done = nullptr;
+    bool rk_wait = false;
     // optional per-kernel timing (mcpg_profile): CUDA events around each launch
     bool prof = false;
     struct Span { const char* name; cudaEvent_t a, b; };

@@ -80,8 +80,25 @@ void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t
         q.rank = q.L.strength + most;
         q.perm = q.rank + most;
     }
+    // after a change of stream, behind the scratch's use on the one before
+    if (!h->rk_done) {
+        if (cudaEventCreateWithFlags(&h->rk_done, cudaEventDisableTiming) != cudaSuccess) {
+            h->rk_done = nullptr;
+            cudaGetLastError();
+            return;
+        }
+    } else if (h->rk_wait && cudaStreamWaitEvent(h->stream, h->rk_done, 0) != cudaSuccess) {
+        return;
+    }
+    h->rk_wait = false;
     if (cudaMemsetAsync(r.cnt, 0, RANKED_COUNTERS * sizeof(unsigned long long), h->stream) != cudaSuccess) return;
     r.on = true;
+}
+
+// Behind every use of the scratch.
+int ranked_used(mcpg_handle* h) {
+    CK(h, cudaEventRecord(h->rk_done, h->stream), "record event");
+    return MCPG_OK;
 }
 
 // One product p (C and/or R of MM_PLAIN / MM_RATIO) with p.A as the owner operand and its lists in
@@ -140,13 +157,13 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
                                           h->stream, &h->launches),
            "ranked witness kernels");
         CK(h, mcpg::launch_maxmin(d, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
-        return MCPG_OK;
+        return ranked_used(h);
     }
     CK(h, mcpg::launch_maxmin(d, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
     CK(h, mcpg::launch_ranked_finish(a, symm ? q.rank : nullptr, symm ? q.rank : nullptr, p.rows, p.cols, p.C, p.ldc,
                                      p.E, p.lde, mode == mcpg::MM_RATIO ? p.R : nullptr, p.ldr, h->stream, &h->launches),
        "ranked finish kernel");
-    return MCPG_OK;
+    return ranked_used(h);
 }
 
 int maxmin_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb, int64_t rows, int64_t cols,
@@ -302,6 +319,7 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
             CK(h, mcpg::launch_ranked_dpi(r, q.rank, p.tol_mult, out, ldo, mask, n, gone, gone + 1, h->stream,
                                           &h->launches),
                "ranked DPI kernels");
+            if ((rc = ranked_used(h))) return rc;
         }
         unsigned long long got[3] = {0, 0, 0};  // NaN seen, pending, removed
         CK(h, cudaMemcpyAsync(got, rk.cnt, sizeof got, cudaMemcpyDeviceToHost, h->stream), "read counters");

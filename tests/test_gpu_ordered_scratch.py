@@ -61,3 +61,30 @@ def test_captured_products_outlive_the_scratch(built_lib, close):
         for k, w in want.items():
             assert np.array_equal(bits(o[k].cpu().numpy()), bits(w)), k
     h.close()
+
+
+def test_products_on_two_streams(built_lib):
+    """A handle moved to another stream while its product is still pending on the first: neither takes the
+    other's lists."""
+    import torch
+    n = 1000
+    a = [symmetric(n, 10 + i, kind) for i, kind in enumerate(("skewed", "uniform"))]
+    A = [torch.from_numpy(x).cuda() for x in a]
+    C = [torch.empty((n, n), device="cuda") for _ in a]
+    streams = [torch.cuda.Stream() for _ in a]
+    with built_lib.Handle(0) as h:
+        h.maxmin_dev(A[0], A[0], C[0])  # scratch in place
+        h.synchronize()
+        want = [exhaustive(x, x) for x in a]
+        for _ in range(5):
+            for i, s in enumerate(streams):
+                C[i].zero_()
+                s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(streams[0]):
+                torch.cuda._sleep(2_000_000)  # about a millisecond
+            for i, s in enumerate(streams):
+                h.set_stream(s.cuda_stream)
+                h.maxmin_dev(A[i], A[i], C[i])
+            torch.cuda.synchronize()
+            for c, w in zip(C, want):
+                assert np.array_equal(bits(c.cpu().numpy()), bits(w))
