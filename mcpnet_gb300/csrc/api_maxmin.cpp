@@ -319,8 +319,15 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
             CK(h, mcpg::launch_ranked_dpi(r, q.rank, p.tol_mult, out, ldo, mask, n, gone, gone + 1, h->stream,
                                           &h->launches),
                "ranked DPI kernels");
-            if ((rc = ranked_used(h))) return rc;
         }
+        if (!removed && n <= 2 * DPI_K0) {
+            // nothing to read back: the one-phase product runs behind where the device gave up, as the products do
+            p.run_above = r.pending_n; p.run_cap = (unsigned long long)r.pending_cap; p.run_nan = r.nan;
+            PROF(h, "maxmin");
+            CK(h, mcpg::launch_maxmin(p, mcpg::MM_DPI, 1, h->stream, &h->launches), "DPI kernel");
+            return ranked_used(h);
+        }
+        if ((rc = ranked_used(h))) return rc;
         unsigned long long got[3] = {0, 0, 0};  // NaN seen, pending, removed
         CK(h, cudaMemcpyAsync(got, rk.cnt, sizeof got, cudaMemcpyDeviceToHost, h->stream), "read counters");
         CK(h, cudaStreamSynchronize(h->stream), "stream synchronize");

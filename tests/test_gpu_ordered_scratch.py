@@ -88,3 +88,44 @@ def test_products_on_two_streams(built_lib):
             torch.cuda.synchronize()
             for c, w in zip(C, want):
                 assert np.array_equal(bits(c.cpu().numpy()), bits(w))
+
+
+@pytest.mark.parametrize("n", [256, 300, 1024])
+def test_dpi_without_a_count_is_asynchronous_and_captured(built_lib, port, n):
+    """Up to 1,024 genes nothing has to be read back: the call returns while the stream is still busy, on
+    matrices the ordered form settles and on those it gives up on (NaN), and it can be captured."""
+    import torch
+    good = symmetric(n, n)
+    bad = good.copy()
+    bad[5, 7] = bad[7, 5] = np.nan
+    s = torch.cuda.Stream()
+    with built_lib.Handle(0) as h:
+        h.set_stream(s.cuda_stream)
+
+        def dpi(A, out, mask):
+            h._check(h._L.mcpg_dpi_dev(h._h, A.data_ptr(), n, n, 0.1, out.data_ptr(), n, mask.data_ptr(), None), "dpi_dev")
+
+        for a in (good, bad):
+            A = torch.from_numpy(a).cuda()
+            out, mask = torch.empty_like(A), torch.empty((n, n), dtype=torch.uint8, device="cuda")
+            want, wmask = torch.empty_like(A), torch.empty_like(mask)
+            h.dpi_dev(A, want, tol=0.1, mask=wmask)  # with a count
+            dpi(A, out, mask)  # scratch in place, kernels loaded
+            torch.cuda.synchronize()
+            with torch.cuda.stream(s):
+                torch.cuda._sleep(200_000_000)  # about 0.1 s
+            dpi(A, out, mask)
+            assert not s.query()
+            torch.cuda.synchronize()
+            assert torch.equal(mask, wmask) and np.array_equal(bits(out.cpu().numpy()), bits(want.cpu().numpy()))
+        oo, om, _ = port.dpi(good, 0.1)
+        A.copy_(torch.from_numpy(good))
+        g = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g, stream=s):
+            dpi(A, out, mask)
+        out.zero_()
+        mask.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(mask.cpu().numpy(), om) and np.array_equal(bits(out.cpu().numpy()), bits(oo))
