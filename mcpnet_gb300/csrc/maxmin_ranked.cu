@@ -373,8 +373,9 @@ __global__ void __launch_bounds__(OWN * 32) walk_kernel(const RankedArgs a) {
 // One warp per pending output: the other row's list (SYM, or where it was built), then both whole rows.
 template <bool SYM>
 __global__ void __launch_bounds__(256) pending_kernel(const RankedArgs a) {
-    if (gave_up(a)) return;
     const int lane = threadIdx.x & 31;
+    // full_n rises while this runs: one lane's reading decides for the warp, whose votes need all lanes
+    if (__any_sync(FULL, lane == 0 && gave_up(a))) return;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t count = (int64_t)*a.pending_n;
     const bool other = !SYM && a.LX.entries && count > (int64_t)a.lx_above;
