@@ -44,7 +44,7 @@ constexpr int RANKED_COUNTERS = 16;
 // or after the handle is gone.
 void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t k, int lists, bool witness = false) {
     r = Ranked{};
-    if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || rows < 8 || k > 32768 || rows > 50000 || cols > 50000) return;
+    if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || rows < 8 || k > 32768 || rows > mcpg::RANKED_MAX_COLS || cols > mcpg::RANKED_MAX_COLS) return;
     if (capturing(h)) return;
     const int64_t most = std::max(rows, cols), lx = round_up(most, 128);  // either operand may own the lists
     const int64_t pitch = mcpg::ranked_list_cap(k);

@@ -98,6 +98,7 @@ struct RankedArgs {
     unsigned long long* full_n;     // (nullable) pending outputs that no list settled; above full_cap: gave up too
     unsigned long long full_cap;
 };
+constexpr int64_t RANKED_MAX_COLS = 50000;  // the finishing kernels' row buffer: 200,000 of 232,448 bytes
 int ranked_list_cap(int64_t k);
 // skip_diag: entry (i, i) is not listed / -inf in XT
 // only_above (device, nullable): nothing unless it exceeds `above`

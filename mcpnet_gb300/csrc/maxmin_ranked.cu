@@ -870,6 +870,14 @@ __global__ void __launch_bounds__(512) dpi_finish_kernel(const RankedArgs a, con
     if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(removed, cnt);
 }
 
+// The finishing kernels hold a product row of up to RANKED_MAX_COLS columns in shared memory.  The attribute is
+// the process's, and always the same value: with each call's own size, another thread's smaller call between the
+// setting and the launch made the launch fail.
+cudaError_t allow_row_buffer(const void* kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(RANKED_MAX_COLS * sizeof(float)));
+}
+
 int isqrt_ceil(int64_t v) { return (int)ceil(sqrt((double)v)); }
 
 }  // namespace
@@ -939,7 +947,7 @@ cudaError_t launch_ranked_finish(const RankedArgs& a, const int* rrank, const in
     const unsigned g = (unsigned)(rows < 152 * 16 ? rows : 152 * 16);
     if (crank) {
         const size_t smem = (size_t)((cols + 3) / 4 * 4) * sizeof(float);
-        cudaError_t e = cudaFuncSetAttribute(finish_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_row_buffer((const void*)finish_kernel<true>);
         if (e != cudaSuccess) return e;
         finish_kernel<true><<<g, 512, smem, st>>>(a, rrank, crank, (int)rows, (int)cols, C, ldc, E, lde, R, ldr);
     } else {
@@ -961,7 +969,7 @@ cudaError_t launch_ranked_dpi(const RankedArgs& a, const int* rank, double tol_m
     dpi_walk_kernel<<<grid, OWN * 32, 0, st>>>(a, tm, asym);
     dpi_ranked_pending_kernel<<<152 * 8, 256, 0, st>>>(a, tm);
     const size_t smem = (size_t)((a.cols + 3) / 4 * 4) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(dpi_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_row_buffer((const void*)dpi_finish_kernel);
     if (e != cudaSuccess) return e;
     dpi_finish_kernel<<<(unsigned)(a.owners < 152 * 16 ? a.owners : 152 * 16), 512, smem, st>>>(
         a, rank, tm, out, ldo, mask, ldmask, removed);

@@ -129,3 +129,32 @@ def test_dpi_without_a_count_is_asynchronous_and_captured(built_lib, port, n):
         g.replay()
         torch.cuda.synchronize()
         assert np.array_equal(mask.cpu().numpy(), om) and np.array_equal(bits(out.cpu().numpy()), bits(oo))
+
+
+def test_products_of_several_threads(built_lib):
+    """A handle per thread, one with rows that need a large row buffer and three with small ones: no launch
+    sees another thread's buffer size."""
+    import threading
+    import torch
+    errors = []
+
+    def work(n, calls):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()), built_lib.Handle(0) as h:
+                h.set_stream(torch.cuda.current_stream().cuda_stream)
+                A = torch.rand((n, 256), device="cuda")
+                C = torch.empty((n, n), device="cuda")
+                torch.cuda.current_stream().synchronize()
+                for _ in range(calls):
+                    h.maxmin_dev(A, A, C)
+                    h.dpi_dev(C, C, tol=0.1)
+                h.synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(f"{n}: {e}")
+
+    threads = [threading.Thread(target=work, args=a) for a in ((13000, 60), (300, 1500), (301, 1500), (257, 1500))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
