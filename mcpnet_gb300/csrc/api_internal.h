@@ -91,14 +91,7 @@ enum Slot {
     S_DPI_PEND,  // two-phase DPI: outputs the first phase left undecided
     S_TCWORK,    // tensor-core MI: the 2-SM form's tile counters
     S_WK,        // MI adjoint: FP32 weights, gene-bin-major
-    S_RK_XT,     // ranked max-min: the transposed operand
-    S_RK_P,      // ranked max-min: the product in strength order
-    S_RK_L0,     // ranked max-min: candidate lists of the first operand
-    S_RK_L1,     // ranked max-min: candidate lists of the second operand
-    S_RK_LX,     // ranked max-min: candidate lists of a product's other operand
-    S_RK_PEND,   // ranked max-min: pending outputs
-    S_RK_CNT,    // ranked max-min: counters
-    S_RK_K,      // ranked max-min: witnesses in strength order
+    S_RK,        // ranked max-min: everything a call's products use (ranked_begin)
     NSLOTS
 };
 

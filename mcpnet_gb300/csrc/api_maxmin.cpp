@@ -34,43 +34,57 @@ struct Ranked {
     RankedSet set[2], other;
 };
 constexpr int RANKED_COUNTERS = 16;
+constexpr int RANKED_TWO = 1;      // some product of the call has two operands
+constexpr int RANKED_WITNESS = 2;  // and some product wants witnesses
+// Outputs that a product may leave pending.  A pending output that its lists do not settle reads two whole
+// rows; 1/64 of the outputs may, which costs less than the exhaustive product.  A product of two
+// operands lets more outputs pend, since the other operand's lists settle most: the MI matrix of 20,000
+// genes times its own M1 leaves a twentieth.
+int64_t ranked_pending_cap(int64_t outputs, bool two) { return std::max<int64_t>(4096, outputs / (two ? 4 : 64)); }
 
-// Decides whether this call's products (at most rows x cols over k) take the ranked form, and lays out
-// its scratch.  Dense below
+// Decides whether this call's products (at most rows x cols over k, lists of `sets` operands kept) take the
+// ranked form, and lays out its scratch.  Dense below
 // MCPG_RANKED_MIN candidates or rows (the ranked form's six launches cost more than one small
 // product), above the list kernel's 32,768 candidates or the finishing kernel's row buffer, where
 // the scratch cannot be had, and in a stream capture: a graph of the exhaustive form holds no
 // scratch of the handle, so it may be replayed after the scratch has grown, on another stream
 // or after the handle is gone.
-void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t k, int lists, bool witness = false) {
+// One allocation: each costs a new handle's first call 10 to 60 us.
+void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t k, int sets, int what) {
     r = Ranked{};
     if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || rows < 8 || k > 32768 || rows > mcpg::RANKED_MAX_COLS || cols > mcpg::RANKED_MAX_COLS) return;
     if (capturing(h)) return;
+    const bool two = (what & RANKED_TWO) != 0;
     const int64_t most = std::max(rows, cols), lx = round_up(most, 128);  // either operand may own the lists
     const int64_t pitch = mcpg::ranked_list_cap(k);
-    r.cap = std::max<int64_t>(4096, rows * cols / 4);
+    r.cap = ranked_pending_cap(rows * cols, two);
+    const size_t pbytes = (size_t)rows * (size_t)round_up(cols, 128) * sizeof(float);
     const size_t lbytes = (size_t)most * (size_t)pitch * sizeof(uint2) + (size_t)most * 5 * sizeof(int);
-    struct { int slot; size_t bytes; void* p; } need[] = {
-        {S_RK_CNT, RANKED_COUNTERS * sizeof(unsigned long long), nullptr},
-        {S_RK_XT, (size_t)k * (size_t)lx * sizeof(float), nullptr},
-        {S_RK_P, (size_t)rows * (size_t)round_up(cols, 128) * sizeof(float), nullptr},
-        {S_RK_PEND, (size_t)r.cap * sizeof(mcpg::RankedPending), nullptr},
-        {S_RK_L0, lbytes, nullptr},
-        {S_RK_L1, lists > 1 ? lbytes : 0, nullptr},
-        {S_RK_LX, lbytes, nullptr},
-        {S_RK_K, witness ? (size_t)rows * (size_t)round_up(cols, 128) * sizeof(int) : 0, nullptr},
+    size_t total = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) / 256 * 256;
+        return at;
     };
-    for (auto& q : need)
-        if (q.bytes && scratch(h, q.slot, q.bytes, &q.p) != MCPG_OK) return;
-    r.cnt = (unsigned long long*)need[0].p;
-    r.XT = (float*)need[1].p;
-    r.P = (float*)need[2].p;
-    r.pending = (mcpg::RankedPending*)need[3].p;
-    r.PK = (int*)need[7].p;
+    const size_t at_cnt = place(RANKED_COUNTERS * sizeof(unsigned long long));
+    const size_t at_xt = place((size_t)k * (size_t)lx * sizeof(float));
+    const size_t at_p = place(pbytes);
+    const size_t at_pend = place((size_t)r.cap * sizeof(mcpg::RankedPending));
+    size_t at_list[3];
+    for (int s = 0; s < 3; ++s) at_list[s] = place(s < sets || (s == 2 && two) ? lbytes : 0);
+    const size_t at_k = place(what & RANKED_WITNESS ? pbytes : 0);
+    void* base;
+    if (scratch(h, S_RK, total, &base) != MCPG_OK) return;
+    char* const b = (char*)base;
+    r.cnt = (unsigned long long*)(b + at_cnt);
+    r.XT = (float*)(b + at_xt);
+    r.P = (float*)(b + at_p);
+    r.pending = (mcpg::RankedPending*)(b + at_pend);
+    r.PK = what & RANKED_WITNESS ? (int*)(b + at_k) : nullptr;
     for (int s = 0; s < 3; ++s) {
-        if (s == 1 && lists < 2) continue;
+        if (!(s < sets || (s == 2 && two))) continue;
         RankedSet& q = s == 2 ? r.other : r.set[s];
-        char* p = (char*)need[4 + s].p;
+        char* p = b + at_list[s];
         q.L.entries = (uint2*)p;
         q.L.pitch = pitch;
         p += (size_t)most * (size_t)pitch * sizeof(uint2);
@@ -134,11 +148,8 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     a.ldp = round_up(swap ? a.owners : a.cols, 128);
     a.direct = symm || !swap;
     a.mirror = symm || swap;
-    // A pending output that its lists do not settle reads two whole rows; 1/64 of the outputs may, which costs
-    // less than the exhaustive product.  A product of two operands lets more outputs pend, since the other
-    // operand's lists settle most: the MI matrix of 20,000 genes times its own M1 leaves a twentieth.
     const int64_t outputs = (int64_t)a.owners * a.cols;
-    a.pending = r.pending; a.pending_cap = std::min(r.cap, std::max<int64_t>(4096, outputs / (symm ? 64 : 4)));
+    a.pending = r.pending; a.pending_cap = std::min(r.cap, ranked_pending_cap(outputs, !symm));
     if (!symm) {
         a.full_n = r.cnt + r.used++;
         a.full_cap = (unsigned long long)std::max<int64_t>(4096, outputs / 64);
@@ -189,7 +200,7 @@ int maxmin_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int6
     p.rows = rows; p.cols = cols; p.k_len = k;
     p.C = C; p.ldc = ldc;
     Ranked r;
-    ranked_begin(h, r, rows, cols, k, 1);
+    ranked_begin(h, r, rows, cols, k, 1, symm ? 0 : RANKED_TWO);
     return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, symm, false);
 }
 
@@ -207,7 +218,7 @@ int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len
     if (rc) return rc;
     const int64_t ldt = round_up(n, 32);
     Ranked rk;
-    ranked_begin(h, rk, n, n, n, path_len == 4 ? 2 : 1);
+    ranked_begin(h, rk, n, n, n, path_len == 4 ? 2 : 1, path_len == 3 ? RANKED_TWO : 0);
     mcpg::MaxminParams p{};
     p.rows = n; p.cols = n; p.k_len = n;
     if (path_len == 2) {
@@ -297,7 +308,7 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
     p.removed = cnt_removed;
     // Candidates in descending order (maxmin_ranked.cu); when that gives up, the forms below.
     Ranked rk;
-    ranked_begin(h, rk, n, n, n, 1);
+    ranked_begin(h, rk, n, n, n, 1, 0);
     if (rk.on) {
         RankedSet& q = rk.set[0];
         mcpg::RankedArgs r{};
@@ -307,7 +318,7 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
         r.XT = rk.XT; r.ldt = round_up(n, 128);
         r.P = rk.P; r.ldp = round_up(n, 128);
         r.direct = r.mirror = 1;
-        r.pending = rk.pending; r.pending_cap = std::max<int64_t>(4096, n * n / 64);
+        r.pending = rk.pending; r.pending_cap = rk.cap;
         r.nan = rk.cnt; r.pending_n = rk.cnt + 1;
         unsigned long long* gone = rk.cnt + 2;
         {
@@ -466,8 +477,9 @@ int maxmin_masked_dev(mcpg_handle* h, const float* A, int64_t lda, const float* 
         p.A = (const float*)a; p.lda = ldk; p.B = bb; p.ldb = lb; p.k_len = k;
     }
     Ranked r;
-    ranked_begin(h, r, rows, cols, p.k_len, 1);
-    return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, same && ts.pm_inf, false);
+    const bool symm = same && ts.pm_inf;
+    ranked_begin(h, r, rows, cols, p.k_len, 1, symm ? 0 : RANKED_TWO);
+    return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, symm, false);
 }
 
 // compute_mcp{2,3,4}_tfs (mcpnet_helper.hpp:209-243, 281-333, 367-434):
@@ -574,7 +586,7 @@ int maxmins_tf_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, const
         CK(h, mcpg::launch_gather(TG, ldt, nullptr, (const int*)idx, t, t, (float*)tt, lk, h->stream, &h->launches),
            "gather kernel");
         Ranked rk;
-        ranked_begin(h, rk, t, n, t, 2);
+        ranked_begin(h, rk, t, n, t, 2, RANKED_TWO);
         mcpg::MaxminParams p{};
         p.rows = t; p.cols = n; p.k_len = t;
         p.A = (const float*)tt; p.lda = lk; p.B = (const float*)ag; p.ldb = lk;
@@ -783,7 +795,7 @@ int maxmin_witness_dev(mcpg_handle* h, const float* A, int64_t lda, const float*
     p.A = a; p.lda = la; p.B = b; p.ldb = lb; p.rows = rows; p.cols = cols; p.k_len = k;
     p.C = C; p.ldc = ldc; p.K = K; p.ldk = ldk;
     Ranked r;
-    ranked_begin(h, r, rows, cols, k, 1, true);
+    ranked_begin(h, r, rows, cols, k, 1, RANKED_WITNESS | (symm ? 0 : RANKED_TWO));
     return ranked_product(h, r, 0, p, mcpg::MM_WITNESS, symm, false);
 }
 
@@ -841,7 +853,7 @@ int maxmins_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float* M
         m1 = (float*)p;
     }
     Ranked rk;
-    ranked_begin(h, rk, n, n, n, M3 || R4 ? 2 : 1);
+    ranked_begin(h, rk, n, n, n, M3 || R4 ? 2 : 1, M2 || R3 ? RANKED_TWO : 0);
     mcpg::MaxminParams p{};
     p.rows = n; p.cols = n; p.k_len = n;
     p.A = a; p.lda = la; p.B = a; p.ldb = la; p.C = m1; p.ldc = l1; p.E = a; p.lde = la; p.R = R2; p.ldr = ldr2;

@@ -158,3 +158,30 @@ def test_products_of_several_threads(built_lib):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("call", ["maxmin", "dpi", "mcp4", "maxmin_two", "witness"])
+def test_scratch_is_what_the_call_can_use(built_lib, call):
+    """The transposed operand, the product, the lists and the pending outputs that the call's kind may leave
+    (1/64 of the outputs, with two operands 1/4), and nothing for the forms it does not take."""
+    import torch
+    n = 4096
+    A, B, C = (torch.rand((n, n), device="cuda") for _ in range(3))
+    K = torch.empty((n, n), dtype=torch.int32, device="cuda")
+    lists = n * (4 * 64 * 8 + 5 * 4)
+    two = call == "maxmin_two"
+    want = 2 * 4 * n * n + (1 + (call == "mcp4") + two) * lists + n * n // (4 if two else 64) * 12
+    want += 4 * n * n * (call in ("mcp4", "witness"))  # M1; the witnesses
+    with built_lib.Handle(0) as h:
+        h.set_stream(torch.cuda.current_stream().cuda_stream)
+        tiny = torch.rand((256, 256), device="cuda")
+        run = {"maxmin": lambda a, b: h.maxmin_dev(a, a, C), "dpi": lambda a, b: h.dpi_dev(a, C),
+               "mcp4": lambda a, b: h.mcp_dev(a, 4, M=C), "maxmin_two": lambda a, b: h.maxmin_dev(a, b, C),
+               "witness": lambda a, b: h.maxmin_witness_dev(a, a, C, K)}[call]
+        run(tiny, tiny.clone())  # kernels loaded
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        run(A, B)
+        torch.cuda.synchronize()
+        used = before - torch.cuda.mem_get_info()[0]
+    assert used <= want + (8 << 20), (used, want)
