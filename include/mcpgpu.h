@@ -554,6 +554,10 @@ MCPG_API int mcpg_last_host_access(const mcpg_handle* h);
  * handle fail with MCPG_ERR_OOM (exercises the error path without a GPU fault). */
 MCPG_API int mcpg_test_fail_allocs(mcpg_handle* h, int count);
 
+/* ---- testing hook: let this handle hold at most `bytes` of device scratch (0: no
+ * limit), as on a device that is nearly full. */
+MCPG_API int mcpg_test_limit_scratch(mcpg_handle* h, int64_t bytes);
+
 /* ---- testing hook: the next tensor-core MI launch of this handle (precision
  * BF16 / FP16 / BF16X3 / FP16X3 / BF16F8) gives every barrier wait a limit of
  * wait_ns nanoseconds (1e3..2e9; the default limit is 2 s), and with starve != 0

@@ -46,6 +46,7 @@ ABI = [
     ("mcpg_synchronize", C.c_int, [_vp]),
     ("mcpg_kernel_launches", C.c_int64, [_vp]),
     ("mcpg_test_fail_allocs", C.c_int, [_vp, C.c_int]),
+    ("mcpg_test_limit_scratch", C.c_int, [_vp, _i64]),
     ("mcpg_test_tc_timeout", C.c_int, [_vp, _i64, C.c_int]),
     ("mcpg_profile", C.c_int, [_vp, C.c_int]),
     ("mcpg_profile_report", C.c_int64, [_vp, C.c_char_p, C.c_int64]),
@@ -277,6 +278,10 @@ class Handle:
 
     def fail_next_allocs(self, count: int):
         self._check(self._L.mcpg_test_fail_allocs(self._h, count), "test_fail_allocs")
+
+    def limit_scratch(self, nbytes: int):
+        """Testing hook: hold at most nbytes of device scratch (0: no limit)."""
+        self._check(self._L.mcpg_test_limit_scratch(self._h, int(nbytes)), "test_limit_scratch")
 
     def test_tc_timeout(self, wait_ns: int, starve: bool = True):
         """Testing hook: the next tensor-core MI launch waits at most wait_ns per barrier

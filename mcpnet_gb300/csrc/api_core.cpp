@@ -135,6 +135,13 @@ int mcpg_test_fail_allocs(mcpg_handle* h, int count) {
     return MCPG_OK;
 }
 
+int mcpg_test_limit_scratch(mcpg_handle* h, int64_t bytes) {
+    if (!h) return MCPG_ERR_ARG;
+    if (bytes < 0) return fail(h, MCPG_ERR_ARG, "test_limit_scratch: negative size");
+    h->alloc_limit = (size_t)bytes;
+    return MCPG_OK;
+}
+
 int mcpg_test_tc_timeout(mcpg_handle* h, int64_t wait_ns, int starve) {
     if (!h) return MCPG_ERR_ARG;
     if (wait_ns < 1000 || wait_ns > (int64_t)mcpg::TC_WAIT_NS_DEFAULT)

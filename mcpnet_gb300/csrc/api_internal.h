@@ -108,6 +108,7 @@ struct mcpg_handle {
     void* buf[NSLOTS] = {};
     size_t cap[NSLOTS] = {};
     int fail_allocs = 0;  // test hook: number of upcoming scratch allocations to fail
+    size_t alloc_limit = 0;  // test hook: bytes of scratch this handle may hold (0: what the device has)
     mcpg::TcWaitHook tc_hook;  // test hook: wait limit / starved producers of the next tensor-core MI launch
     bool tc_hook_armed = false;
     // host MI: a second stream copies finished row slabs back while later slabs compute
@@ -155,24 +156,41 @@ inline bool capturing(mcpg_handle* h) {
     }
     return cs != cudaStreamCaptureStatusNone;
 }
-// Grow-only scratch slot.
+inline cudaError_t scratch_alloc(mcpg_handle* h, size_t bytes, void** p) {
+    if (h->alloc_limit) {
+        size_t held = bytes;
+        for (size_t c : h->cap) held += c;
+        if (held > h->alloc_limit) return cudaErrorMemoryAllocation;
+    }
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+inline void release(mcpg_handle* h, int slot) {
+    if (h->buf[slot]) {
+        cudaStreamSynchronize(h->stream);
+        cudaFree(h->buf[slot]);
+    }
+    h->buf[slot] = nullptr;
+    h->cap[slot] = 0;
+}
+// Grow-only scratch slot.  The ordered max-min form's scratch (S_RK), which every call can do without, makes
+// room for any other slot; a call takes it last, so that none frees it while its own kernels are being enqueued.
 inline int scratch(mcpg_handle* h, int slot, size_t bytes, void** out) {
     if (bytes == 0) bytes = 16;
     if (h->cap[slot] < bytes) {
-        if (h->buf[slot]) {
-            cudaStreamSynchronize(h->stream);
-            cudaFree(h->buf[slot]);
-            h->buf[slot] = nullptr;
-            h->cap[slot] = 0;
-        }
+        release(h, slot);
         if (h->fail_allocs > 0) {
             --h->fail_allocs;
             return fail(h, MCPG_ERR_OOM, "device scratch allocation of %zu bytes failed (injected)", bytes);
         }
         void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, bytes);
+        cudaError_t e = scratch_alloc(h, bytes, &p);
+        if (e == cudaErrorMemoryAllocation && slot != S_RK && h->buf[S_RK]) {
+            release(h, S_RK);
+            e = scratch_alloc(h, bytes, &p);
+        }
         if (e != cudaSuccess) {
-            cudaGetLastError();
             return fail(h, MCPG_ERR_OOM, "device scratch allocation of %zu bytes failed: %s", bytes,
                         cudaGetErrorString(e));
         }

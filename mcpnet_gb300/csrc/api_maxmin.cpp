@@ -217,6 +217,9 @@ int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len
     int rc = aligned_view(h, A, lda, n, n, S_IN0, &a, &la);
     if (rc) return rc;
     const int64_t ldt = round_up(n, 32);
+    void *m1 = nullptr, *m2 = nullptr;
+    if (path_len > 2 && (rc = scratch(h, S_M1, (size_t)(n * ldt) * sizeof(float), &m1))) return rc;
+    if (path_len == 3 && symmetrize && (rc = scratch(h, S_M2, (size_t)(n * ldt) * sizeof(float), &m2))) return rc;
     Ranked rk;
     ranked_begin(h, rk, n, n, n, path_len == 4 ? 2 : 1, path_len == 3 ? RANKED_TWO : 0);
     mcpg::MaxminParams p{};
@@ -227,9 +230,6 @@ int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len
         return ranked_product(h, rk, 0, p, Rout ? mcpg::MM_RATIO : mcpg::MM_PLAIN, true, false);
     }
     // M1 = A (x) A (symmetric)
-    void* m1;
-    rc = scratch(h, S_M1, (size_t)(n * ldt) * sizeof(float), &m1);
-    if (rc) return rc;
     p.A = a; p.lda = la; p.B = a; p.ldb = la; p.C = (float*)m1; p.ldc = ldt;
     if ((rc = ranked_product(h, rk, 0, p, mcpg::MM_PLAIN, true, false))) return rc;
     const float* X1 = (const float*)m1;
@@ -243,9 +243,6 @@ int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len
         q.A = X1; q.lda = ldt; q.B = X1; q.ldb = ldt; sym2 = 1;
     }
     if (path_len == 3 && symmetrize) {
-        void* m2;
-        rc = scratch(h, S_M2, (size_t)(n * ldt) * sizeof(float), &m2);
-        if (rc) return rc;
         q.C = (float*)m2; q.ldc = ldt;
         if ((rc = ranked_product(h, rk, set2, q, mcpg::MM_PLAIN, sym2 != 0, false))) return rc;
         float* sym = Mout;

@@ -185,3 +185,50 @@ def test_scratch_is_what_the_call_can_use(built_lib, call):
         torch.cuda.synchronize()
         used = before - torch.cuda.mem_get_info()[0]
     assert used <= want + (8 << 20), (used, want)
+
+
+def products_case(call, n):
+    """(run(h, operand, outputs), the scratch the exhaustive form needs)."""
+    import torch
+    ld = (n + 31) // 32 * 32
+    nn = 4 * n * ld
+    return {
+        "maxmin": (lambda h, a, o: h.maxmin_dev(a, a, o["C"]), 0),
+        "mcp2": (lambda h, a, o: h.mcp_dev(a, 2, M=o["C"]), 0),
+        "mcp3": (lambda h, a, o: h.mcp_dev(a, 3, M=o["C"]), nn),
+        "mcp3_symmetrized": (lambda h, a, o: h.mcp_dev(a, 3, M=o["C"], symmetrize=True), 2 * nn),
+        "mcp4": (lambda h, a, o: h.mcp_dev(a, 4, M=o["C"]), nn),
+        "maxmins": (lambda h, a, o: h.maxmins_dev(a, M2=o["C"], M3=o["D"]), nn),
+        "witness": (lambda h, a, o: h.maxmin_witness_dev(a, a, o["C"], o["D"].view(torch.int32)), 0),
+    }[call]
+
+
+@pytest.mark.parametrize("call", ["maxmin", "mcp2", "mcp3", "mcp3_symmetrized", "mcp4", "maxmins", "witness"])
+def test_no_call_needs_the_ordered_scratch(built_lib, call):
+    """From the scratch the exhaustive form needs up to all that the ordered one takes, on a new handle and on
+    one whose ordered scratch fills the limit: the same bits."""
+    import torch
+    n = 512
+    run, need = products_case(call, n)
+    A = torch.from_numpy(symmetric(n, 21)).cuda()
+    big = torch.from_numpy(symmetric(1024, 22)).cuda()
+    o = {k: torch.zeros((n, n), device="cuda") for k in "CD"}
+    big_out = torch.empty_like(big)
+    with built_lib.Handle(0) as h:
+        h.set_stream(torch.cuda.current_stream().cuda_stream)
+        run(h, A, o)
+        want = {k: v.cpu() for k, v in o.items()}
+    for limit in [max(need, 1)] + [need + s for s in (1 << 20, 2 << 20, 3 << 20, 4 << 20, 64 << 20)]:
+        for warm in (False, True):
+            with built_lib.Handle(0) as h:
+                h.set_stream(torch.cuda.current_stream().cuda_stream)
+                if warm:  # 1,024 genes' ordered scratch takes most of 12 MB
+                    h.maxmin_dev(big, big, big_out)
+                    limit = max(limit, 12 << 20)
+                h.limit_scratch(limit)
+                for v in o.values():
+                    v.zero_()
+                run(h, A, o)
+                h.synchronize()
+            for k in o:
+                assert torch.equal(o[k].cpu().view(torch.int32), want[k].view(torch.int32)), (limit, warm, k)
