@@ -24,6 +24,36 @@ struct MiPlan {
     int* flag = nullptr;       // tensor-core timeout flag
 };
 
+// FP32 weights in S_W0, sample-major with zero padding.  rows: with what mi_rows_kernel needs (wider padding,
+// entries, flag) behind them, in one allocation: fails without a trace where that cannot be had, or inside a stream
+// capture that would have to allocate it, and the caller takes the form without.
+struct Weights32 {
+    float* wt = nullptr;
+    int64_t genes = 0, ldwt = 0;
+    size_t clear = 0;           // bytes from wt on that have to be zeroed: the weights and the flag
+    float4* ent = nullptr;
+    int* irregular = nullptr;
+};
+int weights32(mcpg_handle* h, int64_t n, int64_t m, int bins, bool rows, Weights32& w) {
+    w = Weights32{};
+    w.genes = rows ? mcpg::mi_rows_genes(n) : round_up(n, 16);
+    w.ldwt = w.genes * bins;
+    const int64_t m_pad = rows ? mcpg::mi_rows_samples(m) : round_up(m, 16);
+    const size_t wbytes = (size_t)(m_pad * w.ldwt) * sizeof(float);  // a multiple of 1,024
+    const size_t total = wbytes + (rows ? 256 + (size_t)(m_pad * w.genes) * sizeof(float4) : 0);
+    if (rows && total > h->cap[S_W0] && capturing(h)) return MCPG_ERR_OOM;
+    void* p;
+    if (int rc = scratch(h, S_W0, total, &p)) return rc;
+    w.wt = (float*)p;
+    w.clear = wbytes;
+    if (rows) {
+        w.irregular = (int*)((char*)p + wbytes);
+        w.ent = (float4*)((char*)p + wbytes + 256);
+        w.clear += sizeof(int);
+    }
+    return MCPG_OK;
+}
+
 int mi_prepare(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx, int bins, int order, int precision,
                float* MI, int64_t ldmi, double* H, MiPlan& pl) {
     if (n < 1 || m < 1) return fail(h, MCPG_ERR_ARG, "bspline_mi: need n >= 1 and m >= 1 (got %lld, %lld)",
@@ -46,30 +76,22 @@ int mi_prepare(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx
     if (precision == MCPG_MI_FP32) {
         if (bins < 2 || bins > 12)
             return fail(h, MCPG_ERR_UNSUPPORTED, "bspline_mi FP32: bins must be 2..12 (got %d)", bins);
-        // three weight rows per sample (mi_rows_kernel), unless its entries do not fit the device
+        Weights32 w;
         bool rows = bins == 10 && order == 3;
-        void *p, *ent = nullptr, *flag = nullptr;
-        if (rows && scratch(h, S_W1, (size_t)(mcpg::mi_rows_samples(m) * mcpg::mi_rows_genes(n)) * sizeof(float4), &ent))
-            rows = false;
-        const int64_t genes = rows ? mcpg::mi_rows_genes(n) : round_up(n, 16);
-        const int64_t ldwt = genes * bins;
-        const int64_t m_pad = rows ? mcpg::mi_rows_samples(m) : round_up(m, 16);
-        if ((rc = scratch(h, S_W0, (size_t)(m_pad * ldwt) * sizeof(float), &p))) return rc;
-        if (rows && (rc = scratch(h, S_SMALL, 64, &flag))) return rc;
-        CK(h, cudaMemsetAsync(p, 0, (size_t)(m_pad * ldwt) * sizeof(float), h->stream), "memset weights");
-        if (rows) CK(h, cudaMemsetAsync(flag, 0, sizeof(int), h->stream), "memset flag");
+        if (rows && weights32(h, n, m, bins, true, w)) rows = false;
+        if (!rows && (rc = weights32(h, n, m, bins, false, w))) return rc;
+        CK(h, cudaMemsetAsync(w.wt, 0, w.clear, h->stream), "memset weights");
         {
             PROF(h, "bspline_weights");
-            CK(h, mcpg::launch_bspline_weights_fp32(X, n, m, ldx, bins, order, (float*)p, ldwt, pl.H, h->stream,
+            CK(h, mcpg::launch_bspline_weights_fp32(X, n, m, ldx, bins, order, w.wt, w.ldwt, pl.H, h->stream,
                                                      &h->launches),
                "bspline weights kernel");
             if (rows)
-                CK(h, mcpg::launch_mi_entries((const float*)p, ldwt, genes, m, (float4*)ent, (int*)flag, h->stream,
-                                              &h->launches),
+                CK(h, mcpg::launch_mi_entries(w.wt, w.ldwt, w.genes, m, w.ent, w.irregular, h->stream, &h->launches),
                    "weight entries kernel");
         }
-        pl.w0 = p; pl.w1 = rows ? ent : nullptr; pl.ldg = genes; pl.irregular = (int*)flag;
-        pl.ld = ldwt;
+        pl.w0 = w.wt; pl.w1 = w.ent; pl.ldg = w.genes; pl.irregular = w.irregular;
+        pl.ld = w.ldwt;
         return MCPG_OK;
     }
     if (bins != 10) return fail(h, MCPG_ERR_UNSUPPORTED, "bspline_mi tensor-core path: only 10 bins (got %d)", bins);

@@ -1,0 +1,52 @@
+"""Device scratch of the FP32 MI and its adjoint: calls that fit without the row-skipping form's
+buffers run without them, with the same bits."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def up(a, b):
+    return (a + b - 1) // b * b
+
+
+@pytest.mark.parametrize("n,m", [(40, 64), (300, 257)])
+def test_fp32_mi_within_the_dense_forms_scratch(built_lib, n, m):
+    import torch
+    X = torch.from_numpy(built_lib.synth_grn(n, m, seed=3)).cuda()
+    MI = torch.empty((n, n), device="cuda")
+    dense = up(m, 16) * up(n, 16) * 10 * 4 + 8 * n  # weights and entropies
+    got = []
+    for limit in (0, dense, dense + (1 << 16)):
+        with built_lib.Handle(0) as h:
+            h.set_stream(torch.cuda.current_stream().cuda_stream)
+            h.limit_scratch(limit)
+            for _ in range(2):
+                MI.zero_()
+                h.bspline_mi_dev(X, MI)
+                got.append(MI.cpu().view(torch.int32))
+    assert all(torch.equal(g, got[0]) for g in got)
+
+
+def test_fp32_mi_captured_in_the_dense_forms_scratch(built_lib):
+    """Scratch in place from a call of another spline order, which has no row-skipping form: a capture does not
+    allocate."""
+    import torch
+    n, m = 64, 100
+    X = torch.from_numpy(built_lib.synth_grn(n, m, seed=4)).cuda()
+    MI, want = torch.empty((n, n), device="cuda"), torch.empty((n, n), device="cuda")
+    s = torch.cuda.Stream()
+    with built_lib.Handle(0) as h:
+        h.bspline_mi_dev(X, want)
+        h.synchronize()
+    with built_lib.Handle(0) as h:
+        h.set_stream(s.cuda_stream)
+        h.bspline_mi_dev(X, MI, 10, 4)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            h.bspline_mi_dev(X, MI)
+        MI.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(MI.view(torch.int32), want.view(torch.int32))
