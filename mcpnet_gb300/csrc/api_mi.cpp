@@ -200,46 +200,45 @@ int mi_bwd_dev(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx
         return fail(h, MCPG_ERR_ARG, "bspline_mi_bwd: need 1 <= order <= bins <= 12, order <= 8");
     if (bins < 2) return fail(h, MCPG_ERR_UNSUPPORTED, "bspline_mi_bwd: bins must be 2..12 (got %d)", bins);
     int rc;
-    void *wt, *wk, *ent = nullptr, *flag = nullptr, *hd, *gs;
-    // three weight rows per sample (mi_rows_kernel), unless its entries do not fit the device
-    bool rows = bins == 10 && order == 3;
-    if (rows && scratch(h, S_W1, (size_t)(mcpg::mi_rows_samples(m) * mcpg::mi_rows_genes(n)) * sizeof(float4), &ent))
-        rows = false;
-    const int64_t genes = rows ? mcpg::mi_rows_genes(n) : round_up(n, 16);
-    const int64_t ldwt = genes * bins;
-    const int64_t m_pad = rows ? mcpg::mi_rows_samples(m) : round_up(m, 16);
-    const int64_t ldk = round_up(m, 128);
-    if ((rc = scratch(h, S_W0, (size_t)(m_pad * ldwt) * sizeof(float), &wt))) return rc;
-    if ((rc = scratch(h, S_WK, (size_t)(n * bins * ldk) * sizeof(float), &wk))) return rc;
-    if (rows && (rc = scratch(h, S_SMALL, 64, &flag))) return rc;
+    const int64_t ldk = round_up(m, 128), lddw = round_up(m, 4), step = 32;
+    Weights32 w;
+    void *wk = nullptr, *hd, *gs, *q = nullptr, *dw = nullptr;
     if ((rc = scratch(h, S_H, (size_t)n * sizeof(double), &hd))) return rc;
     if ((rc = scratch(h, S_GS, (size_t)n * sizeof(float), &gs))) return rc;
-    // slabs of genes j: one for all genes (each pair's Q is then computed once), else 2 GB
-    const int64_t step = 32;
-    int64_t slab = round_up(n, step);
-    void* q = nullptr;
+    // One slab for all genes j (each pair's Q is then computed once) up to MCPG_Q_BYTES (2 GB for the dense
+    // kernel), else slabs of 2 GB.  Where the buffers of the row-skipping form (10 bins / order 3) cannot be had, all
+    // weight rows, and smaller slabs until they can.
+    const bool rows3 = bins == 10 && order == 3;
     auto q_bytes = [&](int64_t g) { return (size_t)(n * bins) * (size_t)round_up(g * bins, 128) * sizeof(float); };
-    if (q_bytes(slab) > (rows ? MCPG_Q_BYTES : (size_t)2 << 30) || scratch(h, S_Q, q_bytes(slab), &q)) {
-        slab = (int64_t)(((size_t)2 << 30) / ((size_t)(n * bins) * bins * sizeof(float))) / step * step;
-        if (slab < step) slab = step;
-        if (slab > round_up(n, step)) slab = round_up(n, step);
-        if ((rc = scratch(h, S_Q, q_bytes(slab), &q))) return rc;
+    const int64_t all = round_up(n, step);
+    int64_t part = (int64_t)(((size_t)2 << 30) / ((size_t)(n * bins) * bins * sizeof(float))) / step * step;
+    part = std::min(std::max(part, step), all);
+    bool rows = rows3;
+    int64_t slab = q_bytes(all) <= (rows ? MCPG_Q_BYTES : (size_t)2 << 30) ? all : part;
+    for (;;) {
+        if (!(rc = weights32(h, n, m, bins, rows, w)) &&
+            !(rc = scratch(h, S_WK, (size_t)(n * bins * ldk) * sizeof(float), &wk)) &&
+            !(rc = scratch(h, S_DW, (size_t)(slab * bins * lddw) * sizeof(float), &dw)) &&
+            !(rc = scratch(h, S_Q, q_bytes(slab), &q)))
+            break;
+        if (rc != MCPG_ERR_OOM || (!rows && slab == step)) return rc;
+        if (!capturing(h))
+            for (int s : {S_W0, S_WK, S_DW, S_Q}) release(h, s);
+        if (slab > part) slab = part;
+        else if (rows) rows = false;
+        else slab = std::max(step, slab / 2 / step * step);
     }
-    const int64_t ldq = round_up(slab * bins, 128), lddw = round_up(m, 4);
-    void* dw;
-    if ((rc = scratch(h, S_DW, (size_t)(slab * bins * lddw) * sizeof(float), &dw))) return rc;
-    CK(h, cudaMemsetAsync(wt, 0, (size_t)(m_pad * ldwt) * sizeof(float), h->stream), "memset weights");
-    if (rows) CK(h, cudaMemsetAsync(flag, 0, sizeof(int), h->stream), "memset flag");
+    const int64_t ldq = round_up(slab * bins, 128);
+    CK(h, cudaMemsetAsync(w.wt, 0, w.clear, h->stream), "memset weights");
     {
         PROF(h, "bspline_weights");
-        CK(h, mcpg::launch_bspline_weights_fp32(X, n, m, ldx, bins, order, (float*)wt, ldwt, (double*)hd, h->stream,
+        CK(h, mcpg::launch_bspline_weights_fp32(X, n, m, ldx, bins, order, w.wt, w.ldwt, (double*)hd, h->stream,
                                                  &h->launches),
            "bspline weights kernel");
         CK(h, mcpg::launch_bspline_weights_k32(X, n, m, ldx, bins, order, (float*)wk, ldk, h->stream, &h->launches),
            "bspline weights kernel");
         if (rows)
-            CK(h, mcpg::launch_mi_entries((const float*)wt, ldwt, genes, m, (float4*)ent, (int*)flag, h->stream,
-                                          &h->launches),
+            CK(h, mcpg::launch_mi_entries(w.wt, w.ldwt, w.genes, m, w.ent, w.irregular, h->stream, &h->launches),
                "weight entries kernel");
     }
     {
@@ -251,11 +250,11 @@ int mi_bwd_dev(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx
         {
             PROF(h, "mi_q");
             if (rows)
-                CK(h, mcpg::launch_mi_q_rows((const float*)wt, ldwt, (const float4*)ent, genes, (const int*)flag, G, ldg,
-                                             n, m, j0, j1, (float*)q, ldq, h->stream, &h->launches),
+                CK(h, mcpg::launch_mi_q_rows(w.wt, w.ldwt, w.ent, w.genes, w.irregular, G, ldg, n, m, j0, j1, (float*)q,
+                                             ldq, h->stream, &h->launches),
                    "MI adjoint Q kernel");
             else
-                CK(h, mcpg::launch_mi_q((const float*)wt, ldwt, G, ldg, n, m, bins, j0, j1, (float*)q, ldq, h->stream,
+                CK(h, mcpg::launch_mi_q(w.wt, w.ldwt, G, ldg, n, m, bins, j0, j1, (float*)q, ldq, h->stream,
                                         &h->launches),
                    "MI adjoint Q kernel");
         }

@@ -50,3 +50,26 @@ def test_fp32_mi_captured_in_the_dense_forms_scratch(built_lib):
         g.replay()
         torch.cuda.synchronize()
         assert torch.equal(MI.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("n,m,order", [(200, 1000, 3), (200, 1000, 4), (600, 64, 3)])
+def test_adjoint_within_less_scratch(built_lib, n, m, order):
+    """From the scratch of one copy of the weights, one slab of Q and dW (the dense form's) down to slabs of 32
+    genes, and up to what the row-skipping form takes.  Every element of Q and of the contraction is the same
+    chain of operations in all of them."""
+    import torch
+    X = torch.from_numpy(built_lib.synth_grn(n, m, seed=6)).cuda()
+    G = torch.randn((n, n), generator=torch.Generator("cuda").manual_seed(1), device="cuda")
+    dX = torch.empty((n, m), device="cuda")
+    w, q = 4 * up(m, 16) * up(n, 16) * 10, 4 * (up(n, 16) * 10) ** 2
+    least = 4 * up(m, 16) * up(n, 16) * 10 + 4 * n * 10 * up(m, 128) + 320 * 4 * up(m, 4) + n * 10 * 384 * 4 + 12 * n
+    got = []
+    for limit in (0, least, (least + 2 * w + q) // 2, 2 * w + q, 3 * w + q, 6 * w + q):
+        with built_lib.Handle(0) as h:
+            h.set_stream(torch.cuda.current_stream().cuda_stream)
+            h.limit_scratch(limit)
+            for _ in range(2):
+                dX.zero_()
+                h.bspline_mi_bwd_dev(X, G, dX, 10, order)
+                got.append(dX.cpu().view(torch.int32))
+    assert all(torch.equal(g, got[0]) for g in got)
