@@ -232,10 +232,8 @@ int mi_bwd_dev(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx
     CK(h, cudaMemsetAsync(w.wt, 0, w.clear, h->stream), "memset weights");
     {
         PROF(h, "bspline_weights");
-        CK(h, mcpg::launch_bspline_weights_fp32(X, n, m, ldx, bins, order, w.wt, w.ldwt, (double*)hd, h->stream,
-                                                 &h->launches),
-           "bspline weights kernel");
-        CK(h, mcpg::launch_bspline_weights_k32(X, n, m, ldx, bins, order, (float*)wk, ldk, h->stream, &h->launches),
+        CK(h, mcpg::launch_bspline_weights_fp32_both(X, n, m, ldx, bins, order, w.wt, w.ldwt, (float*)wk, (double*)hd,
+                                                      h->stream, &h->launches),
            "bspline weights kernel");
         if (rows)
             CK(h, mcpg::launch_mi_entries(w.wt, w.ldwt, w.genes, m, w.ent, w.irregular, h->stream, &h->launches),

@@ -16,7 +16,8 @@
 //   OUT_REF   : W[g*(bins*m+1) + a*m + s] and W[g*(bins*m+1) + bins*m] = (float)H_g
 //               -- the reference's own Transform output row.
 //   OUT_T32   : Wt[s*ldwt + g*bins + a] (sample-major FP32, CUDA-core MI)
-//   OUT_K32   : W[(g*bins + a)*ldw + s] (gene-bin-major FP32, zero-padded to ldw; MI adjoint)
+//   OUT_T32K  : OUT_T32, and out1[(g*bins + a)*ldk + s] (gene-bin-major FP32, ldk = m rounded up to 128,
+//               zero-padded; MI adjoint)
 //   OUT_BF16/OUT_FP16 : Whi/Wlo[(g*bins + a)*ldw + s] (gene-bin-major, K = samples
 //               contiguous, zero-padded to ldw; tcgen05 MI)
 //   OUT_BF16F8 : Whi = bf16(w) * 2^8 (BF16, the layout above), and the E4M3 correction
@@ -57,7 +58,7 @@ struct Knots {
     float r2[KMAX_ORDER + 1][KNOTS_MAX];
 };
 
-enum OutKind { OUT_REF = 0, OUT_T32 = 1, OUT_BF16 = 2, OUT_FP16 = 3, OUT_BF16F8 = 4, OUT_K32 = 5 };
+enum OutKind { OUT_REF = 0, OUT_T32 = 1, OUT_BF16 = 2, OUT_FP16 = 3, OUT_BF16F8 = 4, OUT_T32K = 5 };
 
 void host_knots(int bins, int order, Knots& k) {
     // buildKnotVector<float> (BSplineMI.hpp:35-71): norm_factor in double,
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(WTHREADS) bspline_weights_kernel(const float* 
     const float scale = sh_scale;
     const float offset = (mx > mn) ? mn : 0.0f;
 
+    const int64_t ldk = (m + 127) / 128 * 128;  // OUT_T32K
     CompSum acc[NB];
 
     float w[NB];
@@ -226,12 +228,13 @@ __global__ void __launch_bounds__(WTHREADS) bspline_weights_kernel(const float* 
         if (OUT == OUT_REF) {
             float* W = static_cast<float*>(out0) + g * ((int64_t)bins * m + 1);
             for (int a = 0; a < bins; ++a) W[(int64_t)a * m + s] = w[a];
-        } else if (OUT == OUT_T32) {
+        } else if (OUT == OUT_T32 || OUT == OUT_T32K) {
             float* W = static_cast<float*>(out0) + s * ldo + g * bins;
             for (int a = 0; a < bins; ++a) W[a] = w[a];
-        } else if (OUT == OUT_K32) {
-            float* W = static_cast<float*>(out0) + g * bins * ldo + s;
-            for (int a = 0; a < bins; ++a) W[a * ldo] = w[a];
+            if (OUT == OUT_T32K) {
+                float* K = static_cast<float*>(out1) + g * bins * ldk + s;
+                for (int a = 0; a < bins; ++a) K[a * ldk] = w[a];
+            }
         } else if (OUT == OUT_BF16F8) {
             const int64_t s8 = (s >> 6) * 128 + (s & 63);  // H8 byte of sample s in an HL8 row; L8 at +64
             for (int a = 0; a < bins; ++a) {
@@ -259,9 +262,9 @@ __global__ void __launch_bounds__(WTHREADS) bspline_weights_kernel(const float* 
         }
     }
     // zero the sample padding of the gene-bin-major layouts
-    if (OUT == OUT_K32) {
-        for (int64_t s = m + threadIdx.x; s < ldo; s += blockDim.x)
-            for (int a = 0; a < bins; ++a) static_cast<float*>(out0)[(g * bins + a) * ldo + s] = 0.0f;
+    if (OUT == OUT_T32K) {
+        for (int64_t s = m + threadIdx.x; s < ldk; s += blockDim.x)
+            for (int a = 0; a < bins; ++a) static_cast<float*>(out1)[(g * bins + a) * ldk + s] = 0.0f;
     }
     if (OUT == OUT_BF16F8) {
         for (int64_t s = m + threadIdx.x; s < ldo; s += blockDim.x)
@@ -515,18 +518,19 @@ cudaError_t launch_bspline_weights_fp32(const float* X, int64_t n, int64_t m, in
     return cudaGetLastError();
 }
 
-cudaError_t launch_bspline_weights_k32(const float* X, int64_t n, int64_t m, int64_t ldx, int bins, int order, float* W,
-                                       int64_t ldw, cudaStream_t stream, int64_t* launches) {
+cudaError_t launch_bspline_weights_fp32_both(const float* X, int64_t n, int64_t m, int64_t ldx, int bins, int order,
+                                             float* Wt, int64_t ldwt, float* Wk, double* H, cudaStream_t stream,
+                                             int64_t* launches) {
     if (n <= 0) return cudaSuccess;
     Knots kv;
     host_knots(bins, order, kv);
     if (launches) ++*launches;
     if (bins == 10 && order == 3)
-        bspline_weights_kernel<OUT_K32, 10, 3><<<(unsigned)n, WTHREADS, 0, stream>>>(X, n, m, ldx, bins, order, kv, W,
-                                                                                 nullptr, nullptr, ldw, nullptr);
+        bspline_weights_kernel<OUT_T32K, 10, 3><<<(unsigned)n, WTHREADS, 0, stream>>>(X, n, m, ldx, bins, order, kv, Wt,
+                                                                                  Wk, nullptr, ldwt, H);
     else
-        bspline_weights_kernel<OUT_K32, 0, 0><<<(unsigned)n, WTHREADS, 0, stream>>>(X, n, m, ldx, bins, order, kv, W,
-                                                                               nullptr, nullptr, ldw, nullptr);
+        bspline_weights_kernel<OUT_T32K, 0, 0><<<(unsigned)n, WTHREADS, 0, stream>>>(X, n, m, ldx, bins, order, kv, Wt,
+                                                                                Wk, nullptr, ldwt, H);
     return cudaGetLastError();
 }
 

@@ -188,6 +188,10 @@ cudaError_t launch_copy2d(const float* src, int64_t lds, float* dst, int64_t ldd
 // H[g] (double) = marginal entropy in bits.
 cudaError_t launch_bspline_weights_fp32(const float* X, int64_t n, int64_t m, int64_t ldx, int bins, int order,
                                         float* Wt, int64_t ldwt, double* H, cudaStream_t stream, int64_t* launches);
+// and gene-bin-major too: Wk[(g * bins + a) * ldk + s], ldk = m rounded up to 128, zero for s in [m, ldk).
+cudaError_t launch_bspline_weights_fp32_both(const float* X, int64_t n, int64_t m, int64_t ldx, int bins, int order,
+                                             float* Wt, int64_t ldwt, float* Wk, double* H, cudaStream_t stream,
+                                             int64_t* launches);
 // Gene-bin-major 16-bit weights for tcgen05 (K = samples contiguous):
 //   Whi[(g*bins + a) * ldw + s] = round16(w), Wlo[...] = round16(w - Whi) (Wlo nullable)
 // fmt: 0 = bf16, 1 = fp16.  Columns s in [m, ldw) are written as zero.
@@ -230,9 +234,6 @@ cudaError_t launch_mi_q_rows(const float* Wt, int64_t ldwt, const float4* ent, i
 // multiples of 128 and at least R and S rounded up to that.
 cudaError_t launch_gemm_fp32(const float* A, int64_t lda, const float* B, int64_t ldb, int64_t R, int64_t S, int64_t K,
                              float* C, int64_t ldc, cudaStream_t stream, int64_t* launches);
-// FP32 weights gene-bin-major: W[(gene * bins + a) * ldw + s], zero for s in [m, ldw).
-cudaError_t launch_bspline_weights_k32(const float* X, int64_t n, int64_t m, int64_t ldx, int bins, int order, float* W,
-                                       int64_t ldw, cudaStream_t stream, int64_t* launches);
 // gsum[i] = sum_{j != i} (G[i][j] + G[j][i])
 cudaError_t launch_pair_sums(const float* G, int64_t ldg, int64_t n, float* gsum, cudaStream_t stream,
                              int64_t* launches);

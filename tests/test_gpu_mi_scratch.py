@@ -73,3 +73,19 @@ def test_adjoint_within_less_scratch(built_lib, n, m, order):
                 h.bspline_mi_bwd_dev(X, G, dX, 10, order)
                 got.append(dX.cpu().view(torch.int32))
     assert all(torch.equal(g, got[0]) for g in got)
+
+
+@pytest.mark.parametrize("n,m", [(2, 20), (37, 129)])
+@pytest.mark.parametrize("order,launches", [(3, 6), (4, 5)])
+def test_adjoint_launches(built_lib, port, n, m, order, launches):
+    """Both copies of the weights come from one pass over the samples: weights, pair sums, Q, contraction, dX,
+    and the entries of the row-skipping form."""
+    X = built_lib.synth_grn(n, m, seed=8)
+    G = np.random.default_rng(n).normal(size=(n, n)).astype(np.float32)
+    with built_lib.Handle(0) as h:
+        before = h.kernel_launches
+        got = h.bspline_mi_bwd(X, G, 10, order)
+        assert h.kernel_launches - before == launches
+    want = port.mi_bwd(X.astype(np.float64), G.astype(np.float64), 10, order)
+    # the FP32 adjoint's tolerance elsewhere: 1e-3 of the largest entry
+    assert np.abs(got - want).max() <= 1e-3 * max(np.abs(want).max(), 1e-30)
