@@ -77,7 +77,11 @@ int mi_prepare(mcpg_handle* h, const float* X, int64_t n, int64_t m, int64_t ldx
         if (bins < 2 || bins > 12)
             return fail(h, MCPG_ERR_UNSUPPORTED, "bspline_mi FP32: bins must be 2..12 (got %d)", bins);
         Weights32 w;
-        bool rows = bins == 10 && order == 3;
+        // The row-skipping form reads whole chunks of 64 samples and has a launch more; with few samples the dense
+        // kernel's 16-sample steps win, on fewer genes for longer (dense / row-skipping, us: 64 x 30 24.6 / 26.7, 64 x 60
+        // 28.7 / 26.7, 256 x 40 28.9 / 30.8, 400 x 40 55 / 51, 400 x 30 47 / 51, 600 x 30 72 / 70, 1,000 x 20
+        // 162 / 140, 1,000 x 10 127 / 143, 4,000 x 10 1,519 / 1,653).
+        bool rows = bins == 10 && order == 3 && m > (n < 300 ? 48 : n < 600 ? 32 : 16);
         if (rows && weights32(h, n, m, bins, true, w)) rows = false;
         if (!rows && (rc = weights32(h, n, m, bins, false, w))) return rc;
         CK(h, cudaMemsetAsync(w.wt, 0, w.clear, h->stream), "memset weights");

@@ -89,3 +89,21 @@ def test_adjoint_launches(built_lib, port, n, m, order, launches):
     want = port.mi_bwd(X.astype(np.float64), G.astype(np.float64), 10, order)
     # the FP32 adjoint's tolerance elsewhere: 1e-3 of the largest entry
     assert np.abs(got - want).max() <= 1e-3 * max(np.abs(want).max(), 1e-30)
+
+
+@pytest.mark.parametrize("n,m,launches", [(1, 1, 2), (8, 48, 2), (8, 49, 3), (299, 48, 2), (299, 49, 3), (300, 32, 2),
+                                          (300, 33, 3), (599, 32, 2), (600, 16, 2), (600, 17, 3)])
+def test_few_samples_take_the_dense_form(built_lib, n, m, launches):
+    """At the rule's edges: weights and contraction, or with entries between; the bits of the dense kernel."""
+    import torch
+    X = torch.from_numpy(built_lib.synth_grn(n, m, seed=9)).cuda()
+    MI, want = torch.empty((n, n), device="cuda"), torch.empty((n, n), device="cuda")
+    with built_lib.Handle(0) as h:
+        h.set_stream(torch.cuda.current_stream().cuda_stream)
+        before = h.kernel_launches
+        h.bspline_mi_dev(X, MI)
+        assert h.kernel_launches - before == launches
+    rc = built_lib.lib().mcpg_bspline_mi_fp32_noalloc(X.data_ptr(), n, m, m, 10, 3, want.data_ptr(), n, None,
+                                                      torch.cuda.current_stream().cuda_stream)
+    assert rc == built_lib.OK
+    assert torch.equal(MI.view(torch.int32), want.view(torch.int32))
