@@ -224,7 +224,9 @@ __device__ __noinline__ double ap_flush(const uint32_t* nxy, const uint32_t* nxn
     return sum;
 }
 
-__global__ void __launch_bounds__(AP_WARPS * 32, 4) ap_mi_kernel(ApArgs a) {
+// UN: samples per lane whose loads and sums a window scan keeps in flight, MINB: blocks per SM (launch_ap_mi).
+template <int UN, int MINB>
+__global__ void __launch_bounds__(AP_WARPS * 32, MINB) ap_mi_kernel(ApArgs a) {
     extern __shared__ __align__(16) unsigned char ap_smem[];
     __shared__ int s_i;
     __shared__ int s_next_j;
@@ -357,7 +359,7 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 4) ap_mi_kernel(ApArgs a) {
                 if (nq >= 32) flush();
                 continue;
             }
-#pragma unroll 4
+#pragma unroll(UN < 4 ? 4 : UN)
             for (int k = lane; k < m; k += 32) xg[k] = xr[oY[k]] & 0x3fffu;
             __syncwarp();
             bool broken = false;
@@ -403,8 +405,28 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 4) ap_mi_kernel(ApArgs a) {
                         // per y half: samples left of mx, and in the window
                         auto scan = [&](int from, int to, uint32_t& low, uint32_t& high) {
                             uint32_t l = 0, all = 0;
+                            int k = from + lane;
+                            if (UN > 2) {
+                                uint32_t lu[UN] = {}, au[UN] = {};
+#pragma unroll 1
+                                for (; k + 32 * (UN - 1) < to; k += 32 * UN) {
+                                    unsigned x[UN];
+#pragma unroll
+                                    for (int u = 0; u < UN; ++u) x[u] = (unsigned)xg[k + 32 * u] - wv.x1;
+#pragma unroll
+                                    for (int u = 0; u < UN; ++u) {
+                                        lu[u] += x[u] < wl;
+                                        au[u] += x[u] < wa;
+                                    }
+                                }
+#pragma unroll
+                                for (int u = 0; u < UN; ++u) {
+                                    l += lu[u];
+                                    all += au[u];
+                                }
+                            }
 #pragma unroll 2
-                            for (int k = from + lane; k < to; k += 32) {
+                            for (; k < to; k += 32) {
                                 const unsigned x = (unsigned)xg[k] - wv.x1;
                                 l += x < wl;
                                 all += x < wa;
@@ -524,17 +546,21 @@ cudaError_t launch_ap_mi(const uint16_t* xr, const uint16_t* order, const uint16
     if (warps > AP_WARPS) warps = AP_WARPS;
     if (warps < 1) return cudaErrorNotSupported;
     const size_t smem = xr_bytes + (size_t)warps * a.warp_bytes;
-    cudaError_t e = cudaFuncSetAttribute(ap_mi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // With many genes and up to about 2,500 samples four blocks of 64 registers share an SM, and their warps hide a
+    // scan's latencies.  Where the ranks or the genes leave it fewer, a scan has to keep more in flight itself: tied
+    // values, 100 x 16,384 13.9 -> 8.5 ms, 100 x 8,192 4.9 -> 3.5 ms.
+    auto* const kernel = n > 2 * sms && 4 * (smem + 1024) <= 228 * 1024 ? ap_mi_kernel<2, 4> : ap_mi_kernel<8, 2>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ap_mi_kernel, (int)warps * 32, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)warps * 32, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorNotSupported;
     e = cudaMemsetAsync(next_i, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     int64_t grid = (int64_t)sms * per_sm;
     if (grid > n) grid = n;
-    ap_mi_kernel<<<(unsigned)grid, (unsigned)(warps * 32), smem, st>>>(a);
+    kernel<<<(unsigned)grid, (unsigned)(warps * 32), smem, st>>>(a);
     if (launches) ++*launches;
     return cudaGetLastError();
 }

@@ -113,3 +113,14 @@ def test_ap_mi_small_sizes_and_large_tie_groups(gpu, port, m):
     # so few distinct terms that one log2 rounded the other way (log2 3 in an exact zero at m = 3) moves many
     # entries by an ulp: the distance only, not the share of equal entries
     assert_ap_close(gpu.ap_mi_ranks(R), port.ap_mi(R), exact_frac=0.0)
+
+
+@pytest.mark.parametrize("n,m", [(6, 255), (6, 257), (6, 2600), (320, 40), (5, 5000)])
+def test_ap_mi_few_valued_genes(gpu, port, n, m):
+    """Five-valued genes, whose windows scan bands of many samples, around the 256 samples a wide scan takes at a
+    time and on either side of the rule that chooses the scan's width (more genes than two blocks per SM)."""
+    rng = np.random.default_rng(m)
+    x = rng.standard_normal((n, m))
+    x[1::2] += x[0]
+    R = port.ap_ranks(np.floor(2 * x).astype(np.float32))
+    assert_ap_close(gpu.ap_mi_ranks(R), port.ap_mi(R), exact_frac=0.0)
