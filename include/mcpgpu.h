@@ -558,6 +558,14 @@ MCPG_API int mcpg_test_fail_allocs(mcpg_handle* h, int count);
  * limit), as on a device that is nearly full. */
 MCPG_API int mcpg_test_limit_scratch(mcpg_handle* h, int64_t bytes);
 
+/* ---- testing hook: how the last max-min product or DPI of this handle that could take
+ * the ordered form went, waiting for it.  out[0]: 1 if it was enqueued; then [1] NaN
+ * seen, [2] outputs its lists left pending, [3] more than these: it gave up and the
+ * exhaustive kernel ran, [4] pending outputs that no list settled, [5] their limit (0:
+ * none), [6] more pending than these: the other operand's lists were built. */
+#define MCPG_ORDERED_STATS 7
+MCPG_API int mcpg_test_ordered_stats(mcpg_handle* h, int64_t* out);
+
 /* ---- testing hook: the next tensor-core MI launch of this handle (precision
  * BF16 / FP16 / BF16X3 / FP16X3 / BF16F8) gives every barrier wait a limit of
  * wait_ns nanoseconds (1e3..2e9; the default limit is 2 s), and with starve != 0

@@ -47,6 +47,7 @@ ABI = [
     ("mcpg_kernel_launches", C.c_int64, [_vp]),
     ("mcpg_test_fail_allocs", C.c_int, [_vp, C.c_int]),
     ("mcpg_test_limit_scratch", C.c_int, [_vp, _i64]),
+    ("mcpg_test_ordered_stats", C.c_int, [_vp, _vp]),
     ("mcpg_test_tc_timeout", C.c_int, [_vp, _i64, C.c_int]),
     ("mcpg_profile", C.c_int, [_vp, C.c_int]),
     ("mcpg_profile_report", C.c_int64, [_vp, C.c_char_p, C.c_int64]),
@@ -282,6 +283,12 @@ class Handle:
     def limit_scratch(self, nbytes: int):
         """Testing hook: hold at most nbytes of device scratch (0: no limit)."""
         self._check(self._L.mcpg_test_limit_scratch(self._h, int(nbytes)), "test_limit_scratch")
+
+    def ordered_stats(self) -> dict:
+        """Testing hook: how the last product or DPI that could take the ordered form went."""
+        v = (C.c_int64 * 7)()
+        self._check(self._L.mcpg_test_ordered_stats(self._h, v), "test_ordered_stats")
+        return dict(zip(("enqueued", "nan", "pending", "pending_cap", "full", "full_cap", "lists_above"), v))
 
     def test_tc_timeout(self, wait_ns: int, starve: bool = True):
         """Testing hook: the next tensor-core MI launch waits at most wait_ns per barrier

@@ -142,6 +142,24 @@ int mcpg_test_limit_scratch(mcpg_handle* h, int64_t bytes) {
     return MCPG_OK;
 }
 
+int mcpg_test_ordered_stats(mcpg_handle* h, int64_t* out) {
+    int rc = check_handle(h);
+    if (rc) return rc;
+    if (!out) return fail(h, MCPG_ERR_ARG, "test_ordered_stats: null pointer");
+    const auto& l = h->rk_last;
+    const int64_t zero[MCPG_ORDERED_STATS] = {};
+    std::copy(zero, zero + MCPG_ORDERED_STATS, out);
+    if (!l.pending) return MCPG_OK;
+    if ((rc = finish(h))) return rc;
+    unsigned long long v[3] = {0, 0, 0};
+    const unsigned long long* src[3] = {l.nan, l.pending, l.full};
+    for (int i = 0; i < 3; ++i)
+        if (src[i]) CK(h, cudaMemcpy(&v[i], src[i], sizeof v[i], cudaMemcpyDeviceToHost), "read counters");
+    const int64_t r[MCPG_ORDERED_STATS] = {1, (int64_t)v[0], (int64_t)v[1], l.pending_cap, (int64_t)v[2], l.full_cap, l.lists_above};
+    std::copy(r, r + MCPG_ORDERED_STATS, out);
+    return MCPG_OK;
+}
+
 int mcpg_test_tc_timeout(mcpg_handle* h, int64_t wait_ns, int starve) {
     if (!h) return MCPG_ERR_ARG;
     if (wait_ns < 1000 || wait_ns > (int64_t)mcpg::TC_WAIT_NS_DEFAULT)

@@ -122,6 +122,11 @@ struct mcpg_handle {
     // the ordered max-min form's scratch: its last use, and whether the stream was set since
     cudaEvent_t rk_done = nullptr;
     bool rk_wait = false;
+    // test hook: the counters of the last ordered product (device) and their limits
+    struct {
+        const unsigned long long *nan = nullptr, *pending = nullptr, *full = nullptr;
+        int64_t pending_cap = 0, full_cap = 0, lists_above = 0;
+    } rk_last;
     // optional per-kernel timing (mcpg_profile): CUDA events around each launch
     bool prof = false;
     struct Span { const char* name; cudaEvent_t a, b; };
@@ -173,6 +178,7 @@ inline void release(mcpg_handle* h, int slot) {
     }
     h->buf[slot] = nullptr;
     h->cap[slot] = 0;
+    if (slot == S_RK) h->rk_last = {};
 }
 // Grow-only scratch slot.  The ordered max-min form's scratch (S_RK), which every call can do without, makes
 // room for any other slot; a call takes it last, so that none frees it while its own kernels are being enqueued.

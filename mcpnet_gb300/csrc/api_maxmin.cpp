@@ -42,6 +42,18 @@ constexpr int RANKED_WITNESS = 2;  // and some product wants witnesses
 // genes times its own M1 leaves a twentieth.
 int64_t ranked_pending_cap(int64_t outputs, bool two) { return std::max<int64_t>(4096, outputs / (two ? 4 : 64)); }
 
+// Pending outputs of a two-operand product from which on the other operand's lists pay, 0: never.  Per row, a list of k
+// entries costs about 16 + k / 200 ns (bisection and sort: 0.13 ms for 8,192 rows of 512, 45 us for 2,000 of 2,000,
+// 2.1 ms for 20,000 of 20,000).  A pending output reads two rows, about k / 1,000 ns, or with lists about
+// sqrt(k) / 50; an output of the exhaustive product costs about k / 10,000.  So short rows do without lists, up to
+// where reading the pending ones comes near the exhaustive product: 512 factors x 8,192 genes, where 1/58 of M3's
+// outputs pend, took 0.66 ms with lists from 1/256 on and take 0.53.
+int64_t ranked_lists_pay(int64_t outputs, int64_t rows, int64_t k) {
+    const double gain = (double)k / 1000.0 - std::sqrt((double)k) / 50.0;
+    const double even = (double)rows * (16.0 + (double)k / 200.0) / std::max(gain, 1e-3);
+    return even > (double)outputs / 16.0 ? 0 : (int64_t)std::max(even, (double)outputs / 256.0);
+}
+
 // Decides whether this call's products (at most rows x cols over k, lists of `sets` operands kept) take the
 // ranked form, and lays out its scratch.  Dense below
 // MCPG_RANKED_MIN candidates or rows (the ranked form's six launches cost more than one small
@@ -52,6 +64,7 @@ int64_t ranked_pending_cap(int64_t outputs, bool two) { return std::max<int64_t>
 // One allocation: each costs a new handle's first call 10 to 60 us.
 void ranked_begin(mcpg_handle* h, Ranked& r, int64_t rows, int64_t cols, int64_t k, int sets, int what) {
     r = Ranked{};
+    h->rk_last = {};
     if (k < MCPG_RANKED_MIN || cols < MCPG_RANKED_MIN || rows < 8 || k > 32768 || rows > mcpg::RANKED_MAX_COLS || cols > mcpg::RANKED_MAX_COLS) return;
     if (capturing(h)) return;
     const bool two = (what & RANKED_TWO) != 0;
@@ -150,13 +163,17 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     a.mirror = symm || swap;
     const int64_t outputs = (int64_t)a.owners * a.cols;
     a.pending = r.pending; a.pending_cap = std::min(r.cap, ranked_pending_cap(outputs, !symm));
-    if (!symm) {
+    const int64_t lists_above = symm ? 0 : ranked_lists_pay(outputs, a.cols, a.k);
+    if (lists_above) {
+        a.LX = r.other.L; a.lx_above = (unsigned long long)lists_above;
         a.full_n = r.cnt + r.used++;
-        a.full_cap = (unsigned long long)std::max<int64_t>(4096, outputs / 64);
+        a.full_cap = (unsigned long long)std::max(std::max<int64_t>(4096, outputs / 64), lists_above);
+    } else if (!symm) {
+        a.pending_cap = std::min(a.pending_cap, std::max<int64_t>(4096, outputs / 8));
     }
-    a.LX = r.other.L; a.lx_above = (unsigned long long)(outputs / 256);
     a.pending_n = r.cnt + r.used++;
     a.nan = r.cnt;
+    h->rk_last = {a.nan, a.pending_n, a.full_n, a.pending_cap, (int64_t)a.full_cap, lists_above};
     CK(h, mcpg::launch_ranked_walk(a, symm ? 1 : 0, h->stream, &h->launches), "ranked max-min kernel");
     mcpg::MaxminParams d = p;
     d.run_above = a.pending_n; d.run_cap = (unsigned long long)a.pending_cap; d.run_nan = a.nan;
@@ -318,6 +335,7 @@ int dpi_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float tol, f
         r.pending = rk.pending; r.pending_cap = rk.cap;
         r.nan = rk.cnt; r.pending_n = rk.cnt + 1;
         unsigned long long* gone = rk.cnt + 2;
+        h->rk_last = {r.nan, r.pending_n, nullptr, r.pending_cap, 0, 0};
         {
             PROF(h, "dpi");
             CK(h, mcpg::launch_ranked_lists(a, la, n, n, 1, q.L, rk.cnt, h->stream, &h->launches), "lists kernel");

@@ -36,6 +36,8 @@
 #include <float.h>
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -70,12 +72,12 @@ __device__ __forceinline__ float4 ldg4(const float* p) {
     return v;
 }
 
-// One CTA per owner row: the row's keys sit in registers (EPT per thread); a bisection on the
+// One CTA per owner row (LOOP: per several): the row's keys sit in registers (EPT per thread); a bisection on the
 // key counts entries above a pivot until between want and cap are, they are compacted
 // and sorted (bitonic, key then index).  bound[i] = an upper bound of every entry not
 // listed (-inf when all are).  Entries are padded to a multiple of BATCH with -inf.
-template <int EPT>
-__global__ void __launch_bounds__(LIST_TPB) lists_kernel(const float* __restrict__ O, int64_t ldo, int rows, int k,
+template <int EPT, bool LOOP>
+__global__ void __launch_bounds__(LIST_TPB, EPT <= 16 ? 3 : 1) lists_kernel(const float* __restrict__ O, int64_t ldo, int rows, int k,
                                                          int want, int cap, int strength_at, int skip_diag,
                                                          RankedLists L, unsigned long long* any_nan,
                                                          const unsigned long long* only_above,
@@ -85,148 +87,151 @@ __global__ void __launch_bounds__(LIST_TPB) lists_kernel(const float* __restrict
     __shared__ int wcount[LIST_TPB / 32];
     __shared__ int fill;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int i = blockIdx.x;
-    const float* row = O + (int64_t)i * ldo;
-    int key[EPT];
-    bool nan = false;
-    int mn = INT_MAX, mx = INT_MIN;
-#pragma unroll
-    for (int e = 0; e < EPT; ++e) {
-        const int c = tid + e * LIST_TPB;
-        key[e] = INT_MIN;  // below okey(-inf): never counted
-        if (c < k && !(skip_diag && c == i)) {
-            const float v = row[c];
-            nan |= (v != v);
-            key[e] = okey(v);
-            mn = min(mn, key[e]);
-            mx = max(mx, key[e]);
-        }
-    }
-    if (nan) *any_nan = 1;  // NaN has no place in the order: the exhaustive kernel takes the product
-    auto block_sum = [&](int v) {
-        v = __reduce_add_sync(FULL, v);
-        __syncthreads();
-        if (lane == 0) wcount[warp] = v;
-        __syncthreads();
-        int s = lane < LIST_TPB / 32 ? wcount[lane] : 0;
-        return __reduce_add_sync(FULL, s);
-    };
-    auto above = [&](int pivot) {
-        int c = 0;
-#pragma unroll
-        for (int e = 0; e < EPT; ++e) c += key[e] > pivot;
-        return block_sum(c);
-    };
-    {
-        mn = __reduce_min_sync(FULL, mn);
-        mx = __reduce_max_sync(FULL, mx);
-        __shared__ int smn[LIST_TPB / 32], smx[LIST_TPB / 32];
-        if (lane == 0) { smn[warp] = mn; smx[warp] = mx; }
-        __syncthreads();
-        mn = __reduce_min_sync(FULL, lane < LIST_TPB / 32 ? smn[lane] : INT_MAX);
-        mx = __reduce_max_sync(FULL, lane < LIST_TPB / 32 ? smx[lane] : INT_MIN);
-    }
-    // invariant: above(lo) > cap, above(hi) < want
-    int pivot, n_above;
-    const int avail = k - (skip_diag && i < k);  // entries that may be listed
-    if (avail <= cap) {
-        pivot = INT_MIN;  // everything is listed
-        n_above = avail;
-    } else {
-        long long lo = (long long)mn - 1, hi = mx;
-        pivot = mx;
-        n_above = 0;
-        while (hi - lo > 1) {
-            const int mid = (int)(lo + (hi - lo) / 2);
-            const int c = above(mid);
-            if (c > cap) lo = mid;
-            else {
-                hi = mid;
-                pivot = mid;
-                n_above = c;
-                if (c >= want) break;
-            }
-        }
-    }
-    // entries above the pivot, then entries equal to it as far as the list has room
-    if (tid == 0) fill = 0;
-    __syncthreads();
-    for (int pass = 0; pass < 2; ++pass) {
-        if (pass == 1 && (avail <= cap || n_above >= want)) break;
+    int i = blockIdx.x;
+    do {
+        const float* row = O + (int64_t)i * ldo;
+        int key[EPT];
+        bool nan = false;
+        int mn = INT_MAX, mx = INT_MIN;
 #pragma unroll
         for (int e = 0; e < EPT; ++e) {
-            const bool take = key[e] != INT_MIN && (pass == 0 ? key[e] > pivot : key[e] == pivot);
-            const unsigned b = __ballot_sync(FULL, take);
-            if (!b) continue;
-            int base = 0;
-            if (lane == 0) base = atomicAdd(&fill, __popc(b));
-            base = __shfl_sync(FULL, base, 0);
-            const int at = base + __popc(b & ((1u << lane) - 1u));
-            if (take && at < cap)
-                buf[at] = ((unsigned long long)((unsigned)key[e] ^ 0x80000000u) << 32) | (unsigned)(tid + e * LIST_TPB);
-        }
-        __syncthreads();
-    }
-    const int count = min(fill, cap);
-    int p2 = 32;
-    while (p2 < count) p2 <<= 1;
-    for (int t = count + tid; t < p2; t += LIST_TPB) buf[t] = 0;
-    __syncthreads();
-    if (p2 == LIST_TPB) {
-        // one entry per thread: partners less than a warp apart exchange by shuffle, without a barrier (shorter
-        // lists leave warps idle here and sort faster below: 44 against 54 us for 2,000 rows)
-        unsigned long long v = buf[tid];
-        for (int s = 2; s <= LIST_TPB; s <<= 1) {
-            const bool down = (tid & s) == 0;
-            for (int j = s >> 1; j > 0; j >>= 1) {
-                unsigned long long u;
-                if (j >= 32) {
-                    __syncthreads();
-                    buf[tid] = v;
-                    __syncthreads();
-                    u = buf[tid ^ j];
-                } else {
-                    u = __shfl_xor_sync(FULL, v, j);
-                }
-                const bool first = (tid & j) == 0;  // the lower position keeps the larger where descending
-                v = (first == down) ? (u > v ? u : v) : (u < v ? u : v);
+            const int c = tid + e * LIST_TPB;
+            key[e] = INT_MIN;  // below okey(-inf): never counted
+            if (c < k && !(skip_diag && c == i)) {
+                const float v = row[c];
+                nan |= (v != v);
+                key[e] = okey(v);
+                mn = min(mn, key[e]);
+                mx = max(mx, key[e]);
             }
         }
+        if (nan) *any_nan = 1;  // NaN has no place in the order: the exhaustive kernel takes the product
+        auto block_sum = [&](int v) {
+            v = __reduce_add_sync(FULL, v);
+            __syncthreads();
+            if (lane == 0) wcount[warp] = v;
+            __syncthreads();
+            int s = lane < LIST_TPB / 32 ? wcount[lane] : 0;
+            return __reduce_add_sync(FULL, s);
+        };
+        auto above = [&](int pivot) {
+            int c = 0;
+#pragma unroll
+            for (int e = 0; e < EPT; ++e) c += key[e] > pivot;
+            return block_sum(c);
+        };
+        {
+            mn = __reduce_min_sync(FULL, mn);
+            mx = __reduce_max_sync(FULL, mx);
+            __shared__ int smn[LIST_TPB / 32], smx[LIST_TPB / 32];
+            if (lane == 0) { smn[warp] = mn; smx[warp] = mx; }
+            __syncthreads();
+            mn = __reduce_min_sync(FULL, lane < LIST_TPB / 32 ? smn[lane] : INT_MAX);
+            mx = __reduce_max_sync(FULL, lane < LIST_TPB / 32 ? smx[lane] : INT_MIN);
+        }
+        // invariant: above(lo) > cap, above(hi) < want
+        int pivot, n_above;
+        const int avail = k - (skip_diag && i < k);  // entries that may be listed
+        if (avail <= cap) {
+            pivot = INT_MIN;  // everything is listed
+            n_above = avail;
+        } else {
+            long long lo = (long long)mn - 1, hi = mx;
+            pivot = mx;
+            n_above = 0;
+            while (hi - lo > 1) {
+                const int mid = (int)(lo + (hi - lo) / 2);
+                const int c = above(mid);
+                if (c > cap) lo = mid;
+                else {
+                    hi = mid;
+                    pivot = mid;
+                    n_above = c;
+                    if (c >= want) break;
+                }
+            }
+        }
+        // entries above the pivot, then entries equal to it as far as the list has room
+        if (tid == 0) fill = 0;
         __syncthreads();
-        buf[tid] = v;
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass == 1 && (avail <= cap || n_above >= want)) break;
+#pragma unroll
+            for (int e = 0; e < EPT; ++e) {
+                const bool take = key[e] != INT_MIN && (pass == 0 ? key[e] > pivot : key[e] == pivot);
+                const unsigned b = __ballot_sync(FULL, take);
+                if (!b) continue;
+                int base = 0;
+                if (lane == 0) base = atomicAdd(&fill, __popc(b));
+                base = __shfl_sync(FULL, base, 0);
+                const int at = base + __popc(b & ((1u << lane) - 1u));
+                if (take && at < cap)
+                    buf[at] = ((unsigned long long)((unsigned)key[e] ^ 0x80000000u) << 32) | (unsigned)(tid + e * LIST_TPB);
+            }
+            __syncthreads();
+        }
+        const int count = min(fill, cap);
+        int p2 = 32;
+        while (p2 < count) p2 <<= 1;
+        for (int t = count + tid; t < p2; t += LIST_TPB) buf[t] = 0;
         __syncthreads();
-    } else {
-        for (int s = 2; s <= p2; s <<= 1)
-            for (int j = s >> 1; j > 0; j >>= 1) {
-                for (int t = tid; t < p2 / 2; t += LIST_TPB) {
-                    const int x = ((t & ~(j - 1)) << 1) | (t & (j - 1)), y = x | j;
-                    const unsigned long long a = buf[x], b = buf[y];
-                    if ((a < b) == ((x & s) == 0)) {
-                        buf[x] = b;
-                        buf[y] = a;
+        if (p2 == LIST_TPB) {
+            // one entry per thread: partners less than a warp apart exchange by shuffle, without a barrier (shorter
+            // lists leave warps idle here and sort faster below: 44 against 54 us for 2,000 rows)
+            unsigned long long v = buf[tid];
+            for (int s = 2; s <= LIST_TPB; s <<= 1) {
+                const bool down = (tid & s) == 0;
+                for (int j = s >> 1; j > 0; j >>= 1) {
+                    unsigned long long u;
+                    if (j >= 32) {
+                        __syncthreads();
+                        buf[tid] = v;
+                        __syncthreads();
+                        u = buf[tid ^ j];
+                    } else {
+                        u = __shfl_xor_sync(FULL, v, j);
                     }
+                    const bool first = (tid & j) == 0;  // the lower position keeps the larger where descending
+                    v = (first == down) ? (u > v ? u : v) : (u < v ? u : v);
                 }
-                __syncthreads();
             }
-    }
-    const int padded = (count + BATCH - 1) / BATCH * BATCH;
-    uint2* out = L.entries + (int64_t)i * L.pitch;
-    for (int t = tid; t < padded; t += LIST_TPB) {
-        uint2 e = make_uint2(0xff800000u, 0u);  // -inf
-        if (t < count) {
-            const unsigned long long v = buf[t];
-            e.x = __float_as_uint(okey_value((int)((unsigned)(v >> 32) ^ 0x80000000u)));
-            e.y = (unsigned)v;
+            __syncthreads();
+            buf[tid] = v;
+            __syncthreads();
+        } else {
+            for (int s = 2; s <= p2; s <<= 1)
+                for (int j = s >> 1; j > 0; j >>= 1) {
+                    for (int t = tid; t < p2 / 2; t += LIST_TPB) {
+                        const int x = ((t & ~(j - 1)) << 1) | (t & (j - 1)), y = x | j;
+                        const unsigned long long a = buf[x], b = buf[y];
+                        if ((a < b) == ((x & s) == 0)) {
+                            buf[x] = b;
+                            buf[y] = a;
+                        }
+                    }
+                    __syncthreads();
+                }
         }
-        out[t] = e;
-    }
-    if (tid == 0) {
-        const bool all = count == avail;
-        L.count[i] = count;
-        L.bound[i] = all ? -INFINITY : okey_value(pivot);
-        L.strength[i] = strength_at < count ? (int)((unsigned)(buf[strength_at] >> 32) ^ 0x80000000u)
-                                            : (all ? INT_MIN : pivot);
-    }
+        const int padded = (count + BATCH - 1) / BATCH * BATCH;
+        uint2* out = L.entries + (int64_t)i * L.pitch;
+        for (int t = tid; t < padded; t += LIST_TPB) {
+            uint2 e = make_uint2(0xff800000u, 0u);  // -inf
+            if (t < count) {
+                const unsigned long long v = buf[t];
+                e.x = __float_as_uint(okey_value((int)((unsigned)(v >> 32) ^ 0x80000000u)));
+                e.y = (unsigned)v;
+            }
+            out[t] = e;
+        }
+        if (tid == 0) {
+            const bool all = count == avail;
+            L.count[i] = count;
+            L.bound[i] = all ? -INFINITY : okey_value(pivot);
+            L.strength[i] = strength_at < count ? (int)((unsigned)(buf[strength_at] >> 32) ^ 0x80000000u)
+                                                : (all ? INT_MIN : pivot);
+        }
+        i += gridDim.x;
+    } while (LOOP && i < rows);
 }
 
 // rank[i] = position of row i by ascending strength (ties by index), perm = its inverse.
@@ -403,7 +408,7 @@ __global__ void __launch_bounds__(256) pending_kernel(const RankedArgs a) {
             bound = fminf(bound, bj);
             if (open) open = !__any_sync(FULL, okey(acc) >= okey(bound));
         }
-        if (open && a.full_n) {  // both whole rows: only so many of these
+        if (open && other) {  // both whole rows: only so many of these (without lists no more than lx_above pend)
             unsigned long long seen = 0;
             if (lane == 0) seen = atomicAdd(a.full_n, 1ull);
             if (__shfl_sync(FULL, seen, 0) >= a.full_cap) return;
@@ -895,12 +900,16 @@ cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64
     const int cap = ranked_list_cap(k), want = cap * 3 / 4, at = 2 * isqrt_ceil(k);
     if (k > (int64_t)LIST_TPB * 64 || L.pitch < cap) return cudaErrorInvalidValue;
     if (launches) ++*launches;
-    const unsigned g = (unsigned)rows;
-    if (k <= LIST_TPB * 4) lists_kernel<4><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
-    else if (k <= LIST_TPB * 16) lists_kernel<16><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
-    else if (k <= LIST_TPB * 40) lists_kernel<40><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
-    else lists_kernel<64><<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
-    return cudaGetLastError();
+    // a launch that may have nothing to do: few CTAs (8,192 that return at once take 10 us)
+    const unsigned g = (unsigned)(only_above ? std::min<int64_t>(rows, 152 * 4) : rows);
+    auto launch = [&](auto* kernel) {
+        kernel<<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
+        return cudaGetLastError();
+    };
+    if (k <= LIST_TPB * 4) return launch(only_above ? lists_kernel<4, true> : lists_kernel<4, false>);
+    if (k <= LIST_TPB * 16) return launch(only_above ? lists_kernel<16, true> : lists_kernel<16, false>);
+    if (k <= LIST_TPB * 40) return launch(only_above ? lists_kernel<40, true> : lists_kernel<40, false>);
+    return launch(only_above ? lists_kernel<64, true> : lists_kernel<64, false>);
 }
 
 cudaError_t launch_ranked_order(const RankedLists& L, int64_t n, int* rank, int* perm, cudaStream_t st,
@@ -928,8 +937,7 @@ cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t 
     if (e != cudaSuccess) return e;
     if (!symmetric && a.LX.entries) {
         // An owner with many large entries against a row without: only the other row's list settles
-        // that early.  Its lists are built when such pairs are many (their reading costs as much as one
-        // pending output in 256).
+        // that early.  Its lists are built when such pairs are many.
         e = launch_ranked_lists(a.X, a.ldx, a.cols, a.k, 0, a.LX, const_cast<unsigned long long*>(a.nan), st, launches,
                                 a.pending_n, a.lx_above);
         if (e != cudaSuccess) return e;
