@@ -130,9 +130,12 @@ int ranked_used(mcpg_handle* h) {
 
 // One product p (C and/or R of MM_PLAIN / MM_RATIO) with p.A as the owner operand and its lists in
 // set s; swap: p.B owns (its rows carry the lists), which suits an A whose rows have no
-// pronounced largest values.  Falls back to the exhaustive kernel on the device.
-int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p, int mode, bool symm, bool swap) {
-    if (!r.on || r.used + 3 > RANKED_COUNTERS) {
+// pronounced largest values; choose: the device samples outputs and decides (callers that do not know what the
+// operands hold).  Falls back to the exhaustive kernel on the device.
+int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p, int mode, bool symm, bool swap,
+                   bool choose = false) {
+    choose = choose && !symm;
+    if (!r.on || r.used + (choose ? 5 : 3) > RANKED_COUNTERS) {
         PROF(h, mode == mcpg::MM_WITNESS ? "maxmin_witness" : "maxmin");
         CK(h, mcpg::launch_maxmin(p, mode, symm ? 1 : 0, h->stream, &h->launches), "maxmin kernel");
         return MCPG_OK;
@@ -145,16 +148,17 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     a.owners = (int)(swap ? p.cols : p.rows);
     a.cols = (int)(swap ? p.rows : p.cols);
     a.k = (int)p.k_len;
-    if (!q.built) {
+    if (!choose && !q.built) {
         CK(h, mcpg::launch_ranked_lists(a.O, a.ldo, a.owners, a.k, 0, q.L, r.cnt, h->stream, &h->launches), "lists kernel");
         if (symm) CK(h, mcpg::launch_ranked_order(q.L, a.owners, q.rank, q.perm, h->stream, &h->launches), "order kernel");
         q.built = true;
     }
     a.L = q.L;
     a.ldt = round_up(a.cols, 128);
-    CK(h, mcpg::launch_ranked_transpose(a.X, a.ldx, a.cols, a.k, 0, symm ? q.perm : nullptr, r.XT, a.ldt, r.cnt, h->stream,
-                                        &h->launches),
-       "transpose kernel");
+    if (!choose)
+        CK(h, mcpg::launch_ranked_transpose(a.X, a.ldx, a.cols, a.k, 0, symm ? q.perm : nullptr, r.XT, a.ldt, r.cnt,
+                                            h->stream, &h->launches),
+           "transpose kernel");
     a.XT = r.XT;
     a.perm = symm ? q.perm : nullptr;
     a.P = r.P;
@@ -163,7 +167,7 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     a.mirror = symm || swap;
     const int64_t outputs = (int64_t)a.owners * a.cols;
     a.pending = r.pending; a.pending_cap = std::min(r.cap, ranked_pending_cap(outputs, !symm));
-    const int64_t lists_above = symm ? 0 : ranked_lists_pay(outputs, a.cols, a.k);
+    const int64_t lists_above = symm ? 0 : ranked_lists_pay(outputs, choose ? std::max(a.owners, a.cols) : a.cols, a.k);
     if (lists_above) {
         a.LX = r.other.L; a.lx_above = (unsigned long long)lists_above;
         a.full_n = r.cnt + r.used++;
@@ -173,6 +177,12 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     }
     a.pending_n = r.cnt + r.used++;
     a.nan = r.cnt;
+    if (choose) {
+        int* flip = (int*)(r.cnt + r.used++);
+        unsigned long long* sum = r.cnt + r.used++;
+        a.flip = flip;
+        CK(h, mcpg::launch_ranked_choose(a, flip, sum, r.XT, h->stream, &h->launches), "ranked operand choice kernels");
+    }
     h->rk_last = {a.nan, a.pending_n, a.full_n, a.pending_cap, (int64_t)a.full_cap, lists_above};
     CK(h, mcpg::launch_ranked_walk(a, symm ? 1 : 0, h->stream, &h->launches), "ranked max-min kernel");
     mcpg::MaxminParams d = p;
@@ -194,8 +204,9 @@ int ranked_product(mcpg_handle* h, Ranked& r, int s, const mcpg::MaxminParams& p
     return ranked_used(h);
 }
 
+// choose: as in ranked_product; without it A's rows own the lists.
 int maxmin_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb, int64_t rows, int64_t cols,
-               int64_t k, float* C, int64_t ldc) {
+               int64_t k, float* C, int64_t ldc, bool choose = true) {
     if (rows < 0 || cols < 0 || k < 0) return fail(h, MCPG_ERR_ARG, "maxmin: negative size");
     if (rows == 0 || cols == 0) return MCPG_OK;
     if (!A || !B || !C) return fail(h, MCPG_ERR_ARG, "maxmin: null pointer");
@@ -218,7 +229,7 @@ int maxmin_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int6
     p.C = C; p.ldc = ldc;
     Ranked r;
     ranked_begin(h, r, rows, cols, k, 1, symm ? 0 : RANKED_TWO);
-    return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, symm, false);
+    return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, symm, false, choose);
 }
 
 int mcp_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int path_len, int symmetrize, float* Mout,
@@ -451,7 +462,7 @@ int closure_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, int max_
 // A pure TF mask (+-inf) restricts k to the TF columns (gathered, exact); any
 // other mask is folded into A: min(mask, min(a, b)) == min(min(a, mask), b).
 int maxmin_masked_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb, int64_t rows,
-                      int64_t cols, int64_t k, const float* mask, float* C, int64_t ldc) {
+                      int64_t cols, int64_t k, const float* mask, float* C, int64_t ldc, bool choose = true) {
     if (rows < 0 || cols < 0 || k < 0) return fail(h, MCPG_ERR_ARG, "maxmin_masked: negative size");
     if (rows == 0 || cols == 0) return MCPG_OK;
     if (!A || !B || !C || (k > 0 && !mask)) return fail(h, MCPG_ERR_ARG, "maxmin_masked: null pointer");
@@ -494,7 +505,7 @@ int maxmin_masked_dev(mcpg_handle* h, const float* A, int64_t lda, const float* 
     Ranked r;
     const bool symm = same && ts.pm_inf;
     ranked_begin(h, r, rows, cols, p.k_len, 1, symm ? 0 : RANKED_TWO);
-    return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, symm, false);
+    return ranked_product(h, r, 0, p, mcpg::MM_PLAIN, symm, false, choose);
 }
 
 // compute_mcp{2,3,4}_tfs (mcpnet_helper.hpp:209-243, 281-333, 367-434):
@@ -523,8 +534,8 @@ int mcp_tf_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, const flo
     const float* TG = (const float*)tg;
     auto prod = [&](const float* X, int64_t ldx, int64_t rx, const float* Y, int64_t ldy, int64_t ry, bool masked,
                     float* out, int64_t ldo) -> int {
-        if (masked) return maxmin_masked_dev(h, X, ldx, Y, ldy, rx, ry, n, tfs, out, ldo);
-        return maxmin_dev(h, X, ldx, Y, ldy, rx, ry, n, out, ldo);
+        if (masked) return maxmin_masked_dev(h, X, ldx, Y, ldy, rx, ry, n, tfs, out, ldo, false);
+        return maxmin_dev(h, X, ldx, Y, ldy, rx, ry, n, out, ldo, false);
     };
     float* M = Mout;
     int64_t lm = ldm;
@@ -811,7 +822,7 @@ int maxmin_witness_dev(mcpg_handle* h, const float* A, int64_t lda, const float*
     p.C = C; p.ldc = ldc; p.K = K; p.ldk = ldk;
     Ranked r;
     ranked_begin(h, r, rows, cols, k, 1, RANKED_WITNESS | (symm ? 0 : RANKED_TWO));
-    return ranked_product(h, r, 0, p, mcpg::MM_WITNESS, symm, false);
+    return ranked_product(h, r, 0, p, mcpg::MM_WITNESS, symm, false, true);
 }
 
 int maxmin_bwd_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb, int64_t rows,

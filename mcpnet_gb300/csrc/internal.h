@@ -81,6 +81,12 @@ struct RankedPending {
     int32_t o, p;
     float m;
 };
+// The operand that takes another's place where *flip (device, nullable) is 1; nothing runs where it is 2.
+struct RankedOther {
+    const float* O = nullptr; int64_t ldo = 0;
+    int rows = 0;
+    const int* flip = nullptr;
+};
 struct RankedArgs {
     const float* O; int64_t ldo;  // owner operand, owners x k, 16-byte aligned rows
     const float* X; int64_t ldx;  // other operand, cols x k, 16-byte aligned rows
@@ -97,6 +103,7 @@ struct RankedArgs {
     const unsigned long long* nan;  // nonzero: an operand holds a NaN, and it gave up too
     unsigned long long* full_n;     // (nullable) pending outputs that no list settled; above full_cap: gave up too
     unsigned long long full_cap;
+    const int* flip;                // (device, nullable) 1: X's rows own the lists, and O takes X's place
 };
 constexpr int64_t RANKED_MAX_COLS = 50000;  // the finishing kernels' row buffer: 200,000 of 232,448 bytes
 int ranked_list_cap(int64_t k);
@@ -104,12 +111,17 @@ int ranked_list_cap(int64_t k);
 // only_above (device, nullable): nothing unless it exceeds `above`
 cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64_t k, int skip_diag, const RankedLists& L,
                                 unsigned long long* nan, cudaStream_t st, int64_t* launches,
-                                const unsigned long long* only_above = nullptr, unsigned long long above = 0);
+                                const unsigned long long* only_above = nullptr, unsigned long long above = 0,
+                                const RankedOther& alt = {});
 cudaError_t launch_ranked_order(const RankedLists& L, int64_t n, int* rank, int* perm, cudaStream_t st,
                                 int64_t* launches);
 cudaError_t launch_ranked_transpose(const float* X, int64_t ldx, int64_t rows, int64_t k, int skip_diag,
                                     const int* perm, float* XT,
                                     int64_t ldt, unsigned long long* nan, cudaStream_t st, int64_t* launches);
+// Two operands: decides on the device which one's rows own the lists (flip, also a.flip, and sum: zeroed
+// before), then lists and XT of the owner and the other.
+cudaError_t launch_ranked_choose(const RankedArgs& a, int* flip, unsigned long long* sum, float* XT, cudaStream_t st,
+                                 int64_t* launches);
 // symmetric: O == X, owners in the order of perm, only columns at or after the owner.
 cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t st, int64_t* launches);
 // The DPI filter of O == X (lists and XT with skip_diag): out / mask in gene order, *removed += the

@@ -64,6 +64,38 @@ __device__ __forceinline__ bool gave_up(const RankedArgs& a) {
     return *(const volatile unsigned long long*)a.pending_n > (unsigned long long)a.pending_cap || *a.nan != 0 ||
            (a.full_n && *(const volatile unsigned long long*)a.full_n > a.full_cap);
 }
+// The operands as choose_kernel assigned them: *flip == 1 makes X's rows the owners.
+template <bool FLIP>
+__device__ __forceinline__ RankedArgs oriented(RankedArgs a) {
+    if (FLIP) {
+        if (*a.flip == 1) {
+            const float* o = a.O; a.O = a.X; a.X = o;
+            const int64_t l = a.ldo; a.ldo = a.ldx; a.ldx = l;
+            const int r = a.owners; a.owners = a.cols; a.cols = r;
+            const int d = a.direct; a.direct = a.mirror; a.mirror = d;
+        }
+        a.ldt = (int64_t)(a.cols + COLS - 1) / COLS * COLS;
+    }
+    return a;
+}
+// The owners and columns of this CTA; FLIP: a one-dimensional grid that covers either assignment.
+template <bool FLIP>
+__device__ __forceinline__ bool tile_at(const RankedArgs& a, int& o0, int& p0) {
+    if (FLIP) {
+        const int nb = (a.owners + OWN - 1) / OWN;
+        o0 = (int)(blockIdx.x % nb) * OWN;
+        p0 = (int)(blockIdx.x / nb) * COLS;
+        return p0 < a.cols;
+    }
+    o0 = blockIdx.x * OWN;
+    p0 = blockIdx.y * COLS;
+    return true;
+}
+dim3 tile_grid(const RankedArgs& a) {
+    if (!a.flip) return dim3((unsigned)ceil_div(a.owners, OWN), (unsigned)ceil_div(a.cols, COLS));
+    const int64_t t0 = ceil_div(a.owners, OWN) * ceil_div(a.cols, COLS), t1 = ceil_div(a.cols, OWN) * ceil_div(a.owners, COLS);
+    return dim3((unsigned)std::max(t0, t1));
+}
 // 16 bytes through the read-only path; volatile keeps a batch's loads together and in front
 // of their uses.
 __device__ __forceinline__ float4 ldg4(const float* p) {
@@ -81,13 +113,18 @@ __global__ void __launch_bounds__(LIST_TPB, EPT <= 16 ? 3 : 1) lists_kernel(cons
                                                          int want, int cap, int strength_at, int skip_diag,
                                                          RankedLists L, unsigned long long* any_nan,
                                                          const unsigned long long* only_above,
-                                                         unsigned long long only_cap) {
+                                                         unsigned long long only_cap, const RankedOther alt) {
     if (only_above && *only_above <= only_cap) return;  // uniform: no barrier is passed yet
+    if (alt.flip && *alt.flip) {
+        if (*alt.flip == 2) return;
+        O = alt.O; ldo = alt.ldo; rows = alt.rows;
+    }
     __shared__ unsigned long long buf[LIST_MAX];
     __shared__ int wcount[LIST_TPB / 32];
     __shared__ int fill;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int i = blockIdx.x;
+    if (i >= rows) return;
     do {
         const float* row = O + (int64_t)i * ldo;
         int key[EPT];
@@ -277,13 +314,94 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float* __restrict_
         if (k0 + r < k) XT[(int64_t)(k0 + r) * ldt + p0 + tx] = tile[tx][r];
 }
 
+// The same of the operand that does not own, after choose_kernel (32 x 32 tiles, each CTA several).
+__global__ void __launch_bounds__(256) transpose_chosen_kernel(const RankedArgs a0, float* __restrict__ XT,
+                                                               unsigned long long* any_nan) {
+    __shared__ float tile[32][33];
+    if (*a0.flip == 2) return;
+    const RankedArgs a = oriented<true>(a0);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int nb = (int)(a.ldt / 32), tiles = nb * ((a.k + 31) / 32);
+    for (int b = blockIdx.x; b < tiles; b += gridDim.x) {
+        const int p0 = b % nb * 32, k0 = b / nb * 32;
+#pragma unroll
+        for (int r = ty; r < 32; r += 8) {
+            const int p = p0 + r, c = k0 + tx;
+            const float v = p < a.cols && c < a.k ? a.X[(int64_t)p * a.ldx + c] : INFINITY;
+            if (v != v) *any_nan = 1;
+            tile[r][tx] = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = ty; r < 32; r += 8)
+            if (k0 + r < a.k) XT[(int64_t)(k0 + r) * a.ldt + p0 + tx] = tile[tx][r];
+        __syncthreads();
+    }
+}
+
+// Which operand's rows own the lists: a CTA per sampled output counts the candidates above it in either row.  An
+// output whose owner's list of `cap` entries ends before them pends.  *flip = 1: the samples that pend with O's rows as
+// owners are near what the product may leave pending (`most`), and with X's rows at most half as many do;
+// 2: for a quarter of the samples neither row's list is long enough, more than any product can finish, or with either
+// owner far more would pend than may: the exhaustive kernel is told to run at once.  M1 (x) A used to give up after its walk: 2,000 genes 1.07 ms, against
+// 0.82 exhaustive.
+// sum: zeroed; 16 bits each for the samples that pend with O as owner, with X, with both, and for those done (one
+// atomic: the last CTA has the totals from its result).
+constexpr int SAMPLES = 64, CHOOSE_TPB = 512;
+__global__ void __launch_bounds__(CHOOSE_TPB) choose_kernel(const RankedArgs a, int cap, int most, int* flip,
+                                                           unsigned long long* sum) {
+    __shared__ int part[2][CHOOSE_TPB / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned x = (blockIdx.x + 1u) * 2654435761u, y = (x ^ (x >> 15)) * 2246822519u;
+    const float* ro = a.O + (int64_t)(x % (unsigned)a.owners) * a.ldo;
+    const float* rx = a.X + (int64_t)((y ^ (y >> 13)) % (unsigned)a.cols) * a.ldx;
+    int m = INT_MIN;
+#pragma unroll 4
+    for (int c = threadIdx.x; c < a.k; c += CHOOSE_TPB) m = max(m, okey(fmin2(__ldg(ro + c), __ldg(rx + c))));
+    m = __reduce_max_sync(FULL, m);
+    if (lane == 0) part[0][w] = m;
+    __syncthreads();
+    m = __reduce_max_sync(FULL, lane < CHOOSE_TPB / 32 ? part[0][lane] : INT_MIN);
+    __syncthreads();
+    int no = 0, nx = 0;
+#pragma unroll 4
+    for (int c = threadIdx.x; c < a.k; c += CHOOSE_TPB) {
+        no += okey(__ldg(ro + c)) > m;
+        nx += okey(__ldg(rx + c)) > m;
+    }
+    no = __reduce_add_sync(FULL, no);
+    nx = __reduce_add_sync(FULL, nx);
+    if (lane == 0) {
+        part[0][w] = no;
+        part[1][w] = nx;
+    }
+    __syncthreads();
+    if (w != 0) return;
+    no = __reduce_add_sync(FULL, lane < CHOOSE_TPB / 32 ? part[0][lane] : 0);
+    nx = __reduce_add_sync(FULL, lane < CHOOSE_TPB / 32 ? part[1][lane] : 0);
+    if (lane != 0) return;
+    const unsigned long long one = (unsigned long long)(no > cap) | (unsigned long long)(nx > cap) << 16 |
+                                   (unsigned long long)(no > cap && nx > cap) << 32 | 1ull << 48;
+    const unsigned long long all = atomicAdd(sum, one) + one;
+    if ((all >> 48) != SAMPLES) return;
+    const int po = (int)(all & 0xffff), px = (int)(all >> 16 & 0xffff), both = (int)(all >> 32 & 0xffff);
+    if (both > SAMPLES / 4 || min(po, px) > 2 * most + 4) {
+        *flip = 2;
+        *a.pending_n = (unsigned long long)a.pending_cap + 1;
+    } else if (po > most && 2 * px <= po) {
+        *flip = 1;
+    }
+}
+
 // One warp per (owner, 128 columns).  SYM: owners and columns in strength order, columns
 // at or after the owner only.
-template <bool SYM>
-__global__ void __launch_bounds__(OWN * 32) walk_kernel(const RankedArgs a) {
+template <bool SYM, bool FLIP = false>
+__global__ void __launch_bounds__(OWN * 32) walk_kernel(const RankedArgs a0) {
     __shared__ float tile[OWN][COLS + 4];
-    if (__syncthreads_or(threadIdx.x == 0 && gave_up(a))) return;
-    const int o0 = blockIdx.x * OWN, p0 = blockIdx.y * COLS;
+    if (__syncthreads_or(threadIdx.x == 0 && gave_up(a0))) return;
+    const RankedArgs a = oriented<FLIP>(a0);
+    int o0, p0;
+    if (!tile_at<FLIP>(a, o0, p0)) return;
     if (SYM && p0 + COLS <= o0) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int o = o0 + w, p = p0 + lane * 4;
@@ -376,8 +494,9 @@ __global__ void __launch_bounds__(OWN * 32) walk_kernel(const RankedArgs a) {
 }
 
 // One warp per pending output: the other row's list (SYM, or where it was built), then both whole rows.
-template <bool SYM>
-__global__ void __launch_bounds__(256) pending_kernel(const RankedArgs a) {
+template <bool SYM, bool FLIP = false>
+__global__ void __launch_bounds__(256) pending_kernel(const RankedArgs a0) {
+    const RankedArgs a = oriented<FLIP>(a0);
     const int lane = threadIdx.x & 31;
     // full_n rises while this runs: one lane's reading decides for the warp, whose votes need all lanes
     if (__any_sync(FULL, lane == 0 && gave_up(a))) return;
@@ -481,12 +600,16 @@ __global__ void __launch_bounds__(512) finish_kernel(const RankedArgs a, const i
 // P, those k are the listed ones whose both entries reach P: the lists are walked once more, down to
 // entries below P.  Zeros of either sign are equal here, as in the exhaustive kernel.  Two products with
 // witnesses at 4,096 genes: 36.0 ms (exhaustive, compare and select per candidate) -> 2.2 ms.
-template <bool SYM>
-__global__ void __launch_bounds__(OWN * 32) witness_walk_kernel(const RankedArgs a, int* __restrict__ PK,
+template <bool SYM, bool FLIP = false>
+__global__ void __launch_bounds__(OWN * 32) witness_walk_kernel(const RankedArgs a0, int* __restrict__ PK,
                                                                 unsigned long long* open_n) {
     __shared__ int tile[OWN][COLS + 4];
-    if (__syncthreads_or(threadIdx.x == 0 && gave_up(a))) return;
-    const int o0 = blockIdx.x * OWN, p0 = blockIdx.y * COLS;
+    if (__syncthreads_or(threadIdx.x == 0 &&
+                         (gave_up(a0) || *(const volatile unsigned long long*)open_n > (unsigned long long)a0.pending_cap)))
+        return;
+    const RankedArgs a = oriented<FLIP>(a0);
+    int o0, p0;
+    if (!tile_at<FLIP>(a, o0, p0)) return;
     if (SYM && p0 + COLS <= o0) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int o = o0 + w, p = p0 + lane * 4;
@@ -581,9 +704,10 @@ __global__ void __launch_bounds__(OWN * 32) witness_walk_kernel(const RankedArgs
 // The pending witnesses: one warp each, ascending k, 128 at a time, up to the first that attains C.
 // More of them than the list holds: the first ones are done here, the rest (open_n above the capacity)
 // make the exhaustive kernel run.
-template <bool SYM>
-__global__ void __launch_bounds__(256) witness_pending_kernel(const RankedArgs a, int* __restrict__ PK,
+template <bool SYM, bool FLIP = false>
+__global__ void __launch_bounds__(256) witness_pending_kernel(const RankedArgs a0, int* __restrict__ PK,
                                                               const unsigned long long* open_n) {
+    const RankedArgs a = oriented<FLIP>(a0);
     if (gave_up(a) || *open_n > (unsigned long long)a.pending_cap) return;
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -896,14 +1020,15 @@ int ranked_list_cap(int64_t k) {
 
 cudaError_t launch_ranked_lists(const float* O, int64_t ldo, int64_t rows, int64_t k, int skip_diag, const RankedLists& L,
                                 unsigned long long* nan, cudaStream_t st, int64_t* launches,
-                                const unsigned long long* only_above, unsigned long long above) {
+                                const unsigned long long* only_above, unsigned long long above, const RankedOther& alt) {
     const int cap = ranked_list_cap(k), want = cap * 3 / 4, at = 2 * isqrt_ceil(k);
     if (k > (int64_t)LIST_TPB * 64 || L.pitch < cap) return cudaErrorInvalidValue;
     if (launches) ++*launches;
     // a launch that may have nothing to do: few CTAs (8,192 that return at once take 10 us)
-    const unsigned g = (unsigned)(only_above ? std::min<int64_t>(rows, 152 * 4) : rows);
+    const int64_t most = std::max<int64_t>(rows, alt.flip ? alt.rows : 0);
+    const unsigned g = (unsigned)(only_above ? std::min<int64_t>(most, 152 * 4) : most);
     auto launch = [&](auto* kernel) {
-        kernel<<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above);
+        kernel<<<g, LIST_TPB, 0, st>>>(O, ldo, (int)rows, (int)k, want, cap, at, skip_diag, L, nan, only_above, above, alt);
         return cudaGetLastError();
     };
     if (k <= LIST_TPB * 4) return launch(only_above ? lists_kernel<4, true> : lists_kernel<4, false>);
@@ -928,10 +1053,29 @@ cudaError_t launch_ranked_transpose(const float* X, int64_t ldx, int64_t rows, i
     return cudaGetLastError();
 }
 
+cudaError_t launch_ranked_choose(const RankedArgs& a, int* flip, unsigned long long* sum, float* XT,
+                                 cudaStream_t st, int64_t* launches) {
+    if (launches) *launches += 3;
+    const int most = (int)(SAMPLES * a.pending_cap * 5 / ((int64_t)a.owners * a.cols * 8));
+    choose_kernel<<<SAMPLES, CHOOSE_TPB, 0, st>>>(a, ranked_list_cap(a.k), most, flip, sum);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const RankedOther alt{a.X, a.ldx, a.cols, a.flip};
+    if (launches) --*launches;  // counted below
+    e = launch_ranked_lists(a.O, a.ldo, a.owners, a.k, 0, a.L, const_cast<unsigned long long*>(a.nan), st, launches, nullptr, 0,
+                            alt);
+    if (e != cudaSuccess) return e;
+    const int64_t tiles = ceil_div(std::max(a.owners, a.cols), COLS) * (COLS / 32) * ceil_div(a.k, 32);
+    transpose_chosen_kernel<<<(unsigned)std::min<int64_t>(tiles, 152 * 64), 256, 0, st>>>(
+        a, XT, const_cast<unsigned long long*>(a.nan));
+    return cudaGetLastError();
+}
+
 cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t st, int64_t* launches) {
     if (launches) *launches += 2;
-    dim3 grid((unsigned)ceil_div(a.owners, OWN), (unsigned)ceil_div(a.cols, COLS));
+    const dim3 grid = tile_grid(a);
     if (symmetric) walk_kernel<true><<<grid, OWN * 32, 0, st>>>(a);
+    else if (a.flip) walk_kernel<false, true><<<grid, OWN * 32, 0, st>>>(a);
     else walk_kernel<false><<<grid, OWN * 32, 0, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -939,11 +1083,12 @@ cudaError_t launch_ranked_walk(const RankedArgs& a, int symmetric, cudaStream_t 
         // An owner with many large entries against a row without: only the other row's list settles
         // that early.  Its lists are built when such pairs are many.
         e = launch_ranked_lists(a.X, a.ldx, a.cols, a.k, 0, a.LX, const_cast<unsigned long long*>(a.nan), st, launches,
-                                a.pending_n, a.lx_above);
+                                a.pending_n, a.lx_above, RankedOther{a.O, a.ldo, a.owners, a.flip});
         if (e != cudaSuccess) return e;
     }
     const unsigned g = 152 * 8;
     if (symmetric) pending_kernel<true><<<g, 256, 0, st>>>(a);
+    else if (a.flip) pending_kernel<false, true><<<g, 256, 0, st>>>(a);
     else pending_kernel<false><<<g, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
@@ -989,15 +1134,20 @@ cudaError_t launch_ranked_witness(const RankedArgs& a, int symmetric, const int*
                                   unsigned long long* open_n, int64_t rows, int64_t cols, float* C, int64_t ldc,
                                   int32_t* K, int64_t ldk, cudaStream_t st, int64_t* launches) {
     if (launches) *launches += 3;
-    dim3 grid((unsigned)ceil_div(a.owners, OWN), (unsigned)ceil_div(a.cols, COLS));
+    const dim3 grid = tile_grid(a);
     const unsigned g = (unsigned)(rows < 152 * 16 ? rows : 152 * 16);
     if (symmetric) {
         witness_walk_kernel<true><<<grid, OWN * 32, 0, st>>>(a, PK, open_n);
         witness_pending_kernel<true><<<152 * 8, 256, 0, st>>>(a, PK, open_n);
         witness_finish_kernel<true><<<g, 256, 0, st>>>(a, PK, open_n, rank, (int)rows, (int)cols, C, ldc, K, ldk);
     } else {
-        witness_walk_kernel<false><<<grid, OWN * 32, 0, st>>>(a, PK, open_n);
-        witness_pending_kernel<false><<<152 * 8, 256, 0, st>>>(a, PK, open_n);
+        if (a.flip) {
+            witness_walk_kernel<false, true><<<grid, OWN * 32, 0, st>>>(a, PK, open_n);
+            witness_pending_kernel<false, true><<<152 * 8, 256, 0, st>>>(a, PK, open_n);
+        } else {
+            witness_walk_kernel<false><<<grid, OWN * 32, 0, st>>>(a, PK, open_n);
+            witness_pending_kernel<false><<<152 * 8, 256, 0, st>>>(a, PK, open_n);
+        }
         witness_finish_kernel<false><<<g, 256, 0, st>>>(a, PK, open_n, nullptr, (int)rows, (int)cols, C, ldc, K, ldk);
     }
     return cudaGetLastError();
