@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(AP_WARPS * 32, MINB) ap_mi_kernel(ApArgs a) {
             uint32_t g[4][4];  // [y quartile][x quartile]
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                uint32_t acc = 0;  // four byte counters: a lane sees at most ceil(m / 4 / 32) + ties <= 255 samples
+                uint32_t acc = 0;  // four byte counters, widened before a lane has added 255 samples
                 uint32_t wide = 0, wide2 = 0;
                 int k = bpos[e] + lane;
                 int left = 255;

@@ -222,9 +222,6 @@ cudaError_t launch_bspline_weights_f8(const float* X, int64_t n, int64_t m, int6
 cudaError_t launch_mi_fp32(const float* Wt, int64_t ldwt, const double* H, int64_t n, int64_t m, int bins,
                            float* MI, int64_t ldmi, cudaStream_t stream, int64_t* launches, int64_t gene0 = 0,
                            int64_t gene1 = -1);
-// MI adjoint, slab of gene tiles [tile0, tile0 + tiles) (16 genes each) x all genes:
-// Q[(i - 16*tile0)*bins + a][j*bins + b] = Gs_ij (log2 P_ab + 1/ln 2) [P_ab > 0],
-// Gs_ij = G[i][j] + G[j][i] (i != j), recomputing P from the sample-major weights.
 // The same MI for 10 bins / order 3 (same bits), three weight rows per sample instead of ten.
 // Wt zero-padded to mi_rows_genes(n) genes (ldwt = that * 10) and mi_rows_samples(m) samples;
 // ent: mi_rows_samples(m) x ldg entries, ldg = mi_rows_genes(n); *irregular zeroed before.
@@ -235,6 +232,9 @@ cudaError_t launch_mi_entries(const float* Wt, int64_t ldwt, int64_t ldg, int64_
 cudaError_t launch_mi_rows(const float* Wt, int64_t ldwt, const float4* ent, int64_t ldg, const int* irregular,
                            const double* H, int64_t n, int64_t m, float* MI, int64_t ldmi, int64_t gene0,
                            int64_t gene1, cudaStream_t stream, int64_t* launches);
+// MI adjoint, all genes i x a slab of genes j in [j0, j1), j0 a multiple of 16:
+// Q[i*bins + a][(j - j0)*bins + b] = Gs_ij (log2 P_ab + 1/ln 2) [P_ab > 0],
+// Gs_ij = G[i][j] + G[j][i] (i != j), recomputing P from the sample-major weights.
 cudaError_t launch_mi_q(const float* Wt, int64_t ldwt, const float* G, int64_t ldg, int64_t n, int64_t m, int bins,
                         int64_t j0, int64_t j1, float* Q, int64_t ldq, cudaStream_t stream, int64_t* launches);
 // The same Q from the inputs of launch_mi_rows (j0 a multiple of 32); over all genes j, each
