@@ -626,8 +626,9 @@ def pipeline_run(args, local):
     ldw = -(-m // 64) * 64
     w_bytes = n * m * 4 + 2 * n * b * ldw * 2
     mm_ms = st["mcp234"] * 1e3
-    # executed min/max work: M1 and M3 symmetric (n^3 / 2 triples each), M2 full (n^3)
-    mm_ops_exec = 2.0 * (0.5 + 1.0 + 0.5) * n ** 3
+    # min/max work of the full products: M1 and M3 symmetric (n^3 / 2 triples each), M2 full (n^3)
+    mm_ops_full = 2.0 * (0.5 + 1.0 + 0.5) * n ** 3
+    ordered_note = "the ordered form visits a few percent of the full products' triples, so the fraction can exceed 1"
     stages = {}
     if args.mi_method == "ap":
         stages["ap_mi"] = {"ms": st["mi"] * 1e3, "pairs_per_s": n * (n + 1) / 2 / st["mi"],
@@ -642,11 +643,12 @@ def pipeline_run(args, local):
                            "frac_tensor_issued": {"bf16x3": 3.0, "fp16x3": 3.0, "bf16f8": 2.0, "bf16": 1.0,
                                                   "fp16": 1.0}.get(args.precision, 0.0)
                            * mi_flops * (128 / 120) / (tc_ms / 1e3) / tc_peak}
-    stages["maxmin_M1_M2_M3_with_ratios"] = {"ms": mm_ms, "Gop/s_executed": mm_ops_exec / (mm_ms / 1e3) / 1e9,
-                                             "frac_alu_peak": mm_ops_exec / (mm_ms / 1e3) / alu_peak}
+    stages["maxmin_M1_M2_M3_with_ratios"] = {"ms": mm_ms, "Gop/s_full_products": mm_ops_full / (mm_ms / 1e3) / 1e9,
+                                             "frac_alu_peak_full_products": mm_ops_full / (mm_ms / 1e3) / alu_peak,
+                                             "note": ordered_note}
     dpi_ms = st["dpi"] * 1e3
     stages["dpi"] = {"ms": dpi_ms, "removed": removed[0],
-                     "frac_alu_peak": 2.0 * 0.5 * n ** 3 / (dpi_ms / 1e3) / alu_peak}
+                     "frac_alu_peak_full_products": 2.0 * 0.5 * n ** 3 / (dpi_ms / 1e3) / alu_peak}
     if args.closure:
         cl_ms = st["closure"] * 1e3
         stages["closure"] = {"ms": cl_ms, "iterations": iters,
@@ -670,14 +672,14 @@ def pipeline_run(args, local):
                            "best_aupr": float(pr[best]), "best_auroc": float(roc[best])}
     if args.tfs > 0:
         t = tfst["t"]
-        # executed triples: MCP2 T(x)A; MCP3 A(x)A (symmetric) + T(x)M1; MCP4 A(x)A + T(x)A + M2(x)M1
+        # triples of the full products: MCP2 T(x)A; MCP3 A(x)A (symmetric) + T(x)M1; MCP4 A(x)A + T(x)A + M2(x)M1
         # (every masked product runs over the t TF columns)
         tri = {"mcp_tf": n * n * t + 4.0 * t * t * n, "maxmins_tf": 0.5 * n * n * t + 3.0 * t * t * n,
                "dpi_tf": 0.5 * n ** 3 + 0.5 * n * n * t}
         for key in ("mcp_tf", "maxmins_tf", "dpi_tf"):
             ms_ = st[key] * 1e3
-            stages[key] = {"ms": ms_, "tfs": t, "Gop/s_executed": 2 * tri[key] / (ms_ / 1e3) / 1e9,
-                           "frac_alu_peak": 2 * tri[key] / (ms_ / 1e3) / alu_peak}
+            stages[key] = {"ms": ms_, "tfs": t, "Gop/s_full_products": 2 * tri[key] / (ms_ / 1e3) / 1e9,
+                           "frac_alu_peak_full_products": 2 * tri[key] / (ms_ / 1e3) / alu_peak}
         stages["dpi_tf"]["removed"] = tfst["removed"]
         if not args.no_eval:
             stages["tf_eval_mcp2"] = {"ms": st["tf_eval_mcp2"] * 1e3, "aupr": tfst["mcp2"][0],
