@@ -241,6 +241,10 @@ MCPG_API int mcpg_maxmin_witness(mcpg_handle* h, const float* A, int64_t lda, co
 MCPG_API int mcpg_maxmin_witness_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb,
                                      int64_t rows, int64_t cols, int64_t k_len, float* C, int64_t ldc, int32_t* K,
                                      int64_t ldk);
+/* M1 = A (x) A and M2 = A (x) M1 with their witnesses, A n x n: the bits of two calls above, the lists of A's
+ * rows made once. */
+MCPG_API int mcpg_maxmins_witness_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float* M1, int64_t ld1,
+                                      int32_t* K1, int64_t ldk1, float* M2, int64_t ld2, int32_t* K2, int64_t ldk2);
 MCPG_API int mcpg_maxmin_bwd(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb,
                              int64_t rows, int64_t cols, int64_t k_len, const float* C, int64_t ldc,
                              const float* dC, int64_t lddc, const int32_t* K, int64_t ldk, float* dA, int64_t ldda,

@@ -75,6 +75,8 @@ ABI = [
     ("mcpg_dpi_tf_dev", C.c_int, [_vp, _vp, _i64, _i64, C.c_float, _vp, _vp, _i64, _vp, C.POINTER(C.c_int64)]),
     ("mcpg_closure_dev", C.c_int, [_vp, _vp, _i64, _i64, C.c_int, _vp, _i64, C.POINTER(C.c_int)]),
     ("mcpg_maxmin_witness", C.c_int, [_vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _vp, _i64, _vp, _i64]),
+    ("mcpg_maxmins_witness_dev", C.c_int,
+     [_vp, _vp, _i64, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64]),
     ("mcpg_maxmin_witness_dev", C.c_int, [_vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _vp, _i64, _vp, _i64]),
     ("mcpg_maxmin_bwd", C.c_int, [_vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _vp, _i64, _vp, _i64, _vp, _i64,
                                   _vp, _i64, _vp, _i64]),
@@ -536,11 +538,12 @@ class Handle:
         if witness == "saved":
             K1 = torch.empty((n, n), dtype=torch.int32, device=dev)
             K2 = torch.empty((n, n), dtype=torch.int32, device=dev)
-            self.maxmin_witness_dev(A, A, M1, K1)
-            self.maxmin_witness_dev(A, M1, M2, K2)
+            self._check(self._L.mcpg_maxmins_witness_dev(self._h, self._dp(A), n, self._ld(A), self._dp(M1),
+                                                         self._ld(M1), self._dp(K1), self._ld(K1), self._dp(M2),
+                                                         self._ld(M2), self._dp(K2), self._ld(K2)),
+                        "maxmins_witness_dev")
         else:
-            self.maxmin_dev(A, A, M1)
-            self.maxmin_dev(A, M1, M2)
+            self.maxmins_dev(A, M1=M1, M2=M2)
         self.ratio_dev(A, M2, R)
         L = (coef.to(torch.float64) * R[rows_idx, cols_idx].to(torch.float64)).sum()
         dR = torch.zeros((n, n), **f32)

@@ -825,6 +825,37 @@ int maxmin_witness_dev(mcpg_handle* h, const float* A, int64_t lda, const float*
     return ranked_product(h, r, 0, p, mcpg::MM_WITNESS, symm, false, true);
 }
 
+// Both products with A's rows as owners (M1's have no pronounced largest values), A's lists kept between them.
+int maxmins_witness_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float* M1, int64_t ld1, int32_t* K1,
+                        int64_t ldk1, float* M2, int64_t ld2, int32_t* K2, int64_t ldk2) {
+    if (n < 0) return fail(h, MCPG_ERR_ARG, "maxmins_witness: negative size");
+    if (n == 0) return MCPG_OK;
+    if (!A || !M1 || !K1 || !M2 || !K2) return fail(h, MCPG_ERR_ARG, "maxmins_witness: null pointer");
+    if (lda < n || ld1 < n || ldk1 < n || ld2 < n || ldk2 < n)
+        return fail(h, MCPG_ERR_ARG, "maxmins_witness: leading dimension too small");
+    const float* a;
+    int64_t la, l1 = ld1;
+    int rc = aligned_view(h, A, lda, n, n, S_IN0, &a, &la);
+    if (rc) return rc;
+    float* m1 = M1;
+    if (!aligned16(M1) || (ld1 % 4) != 0) {
+        void* p;
+        l1 = round_up(n, 32);
+        if ((rc = scratch(h, S_M1, (size_t)(n * l1) * sizeof(float), &p))) return rc;
+        m1 = (float*)p;
+    }
+    Ranked r;
+    ranked_begin(h, r, n, n, n, 1, RANKED_WITNESS | RANKED_TWO);
+    mcpg::MaxminParams p{};
+    p.rows = n; p.cols = n; p.k_len = n;
+    p.A = a; p.lda = la; p.B = a; p.ldb = la; p.C = m1; p.ldc = l1; p.K = K1; p.ldk = ldk1;
+    if ((rc = ranked_product(h, r, 0, p, mcpg::MM_WITNESS, true, false))) return rc;
+    p.B = m1; p.ldb = l1; p.C = M2; p.ldc = ld2; p.K = K2; p.ldk = ldk2;
+    if ((rc = ranked_product(h, r, 0, p, mcpg::MM_WITNESS, false, false))) return rc;
+    if (m1 != M1) CK(h, mcpg::launch_copy2d(m1, l1, M1, ld1, n, n, h->stream), "copy2d");
+    return MCPG_OK;
+}
+
 int maxmin_bwd_dev(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb, int64_t rows,
                    int64_t cols, int64_t k, const float* C, int64_t ldc, const float* dC, int64_t lddc,
                    const int32_t* K, int64_t ldk, float* dA, int64_t ldda, float* dB, int64_t lddb) {
@@ -1182,6 +1213,13 @@ int mcpg_maxmin_witness_dev(mcpg_handle* h, const float* A, int64_t lda, const f
     int rc = check_handle(h);
     if (rc) return rc;
     return maxmin_witness_dev(h, A, lda, B, ldb, rows, cols, k, C, ldc, K, ldk);
+}
+
+int mcpg_maxmins_witness_dev(mcpg_handle* h, const float* A, int64_t n, int64_t lda, float* M1, int64_t ld1,
+                             int32_t* K1, int64_t ldk1, float* M2, int64_t ld2, int32_t* K2, int64_t ldk2) {
+    int rc = check_handle(h);
+    if (rc) return rc;
+    return maxmins_witness_dev(h, A, n, lda, M1, ld1, K1, ldk1, M2, ld2, K2, ldk2);
 }
 
 int mcpg_maxmin_witness(mcpg_handle* h, const float* A, int64_t lda, const float* B, int64_t ldb, int64_t rows,
