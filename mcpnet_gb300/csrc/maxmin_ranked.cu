@@ -32,7 +32,7 @@
 // Measured on MI-like matrices (symmetric product with ratio, whole call; exhaustive form ->
 // this one): 20,000 genes 338 -> 18.8 ms (walk 13.5, lists 2.1, finish 1.6, transpose 1.1 ms); M1..M3
 // with ratios at 2,000 genes 1.79 -> 0.46 ms; 300 genes, one product, 71 -> 49 us.  ncu at 8,192 genes: the
-// walk reads 18.9 TB/s from L2, 79 % of what the L1s take in.
+// walk keeps L1 and L2 at 77 % of their throughput, 97 % of its L1 misses hit L2.
 #include <float.h>
 #include <math.h>
 
@@ -343,8 +343,8 @@ __global__ void __launch_bounds__(256) transpose_chosen_kernel(const RankedArgs 
 // output whose owner's list of `cap` entries ends before them pends.  *flip = 1: the samples that pend with O's rows as
 // owners are near what the product may leave pending (`most`), and with X's rows at most half as many do;
 // 2: for a quarter of the samples neither row's list is long enough, more than any product can finish, or with either
-// owner far more would pend than may: the exhaustive kernel is told to run at once.  M1 (x) A used to give up after its walk: 2,000 genes 1.07 ms, against
-// 0.82 exhaustive.
+// owner far more would pend than may: the exhaustive kernel is told to run at once.  M1 (x) A at 2,000 genes takes 0.20
+// ms; from M1's rows it gave up after the walk, 1.07 ms (0.82 exhaustive).  The samples take 5 to 8 us.
 // sum: zeroed; 16 bits each for the samples that pend with O as owner, with X, with both, and for those done (one
 // atomic: the last CTA has the totals from its result).
 constexpr int SAMPLES = 64, CHOOSE_TPB = 512;
@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(256) witness_finish_kernel(const RankedArgs a,
 // output settled as soon as its maximum reaches the threshold or no later entry can.  On MI
 // matrices nearly every pair is decided by its first few entries.  P receives a value
 // on the right side of both orientations' thresholds.  Measured (whole call, tolerance 0.1; the tiled
-// first-phase form -> this one): 20,000 genes 69.4 -> 11.3 ms (walk 6.4, lists 2.1, finish 1.2 ms; 14.8 ms
+// first-phase form -> this one): 20,000 genes 69.4 -> 11.8 ms (walk 6.4, lists 2.1, finish 1.2 ms; 14.8 ms
 // with the thresholds' products in FP64 and gathered for both orientations), 2,000 genes 355 -> 174 us.
 // The threshold (float)(e * tm) with the product in double, mostly without the FP64 pipe (16 clocks of an SM
 // per warp instruction): e times tm as a pair of floats, exact to 2^-45.  Where the rounding to float is
@@ -1048,7 +1048,9 @@ int isqrt_ceil(int64_t v) { return (int)ceil(sqrt((double)v)); }
 int ranked_list_cap(int64_t k) {
     // four square roots of the candidate count cover 99 % of the outputs of the measured matrices
     int64_t c = (4 * (int64_t)isqrt_ceil(k) + 31) / 32 * 32;
-    if (c > LIST_TPB && c <= LIST_TPB + 128) c = LIST_TPB;  // one entry per thread of the sort (k up to 25,600)
+    // one entry per thread of the sort (k up to 25,600): the DPI gains throughout (24,000 genes 17.8 ms, 18.6 with 640
+    // entries), products up to about 21,000 (22.2 and 22.0 ms; at 24,000 32.4 and 29.9)
+    if (c > LIST_TPB && c <= LIST_TPB + 128) c = LIST_TPB;
     return (int)(c > LIST_MAX ? LIST_MAX : c);
 }
 

@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 // Per 32 pairs and sample: 1,280 B of j weights and a broadcast entry of i from shared
 // memory (12 clocks with the staging writes), 7.5 clocks of packed multiply-adds.  Measured
 // (weights excluded): 2,000 x 2,000 16.7 -> 7.0 ms, 4,000 x 2,000 66.2 -> 27.0 ms, 500 x 500
-// 346 -> 151 us; the shared-memory pipe is 72 % busy, the rest are branch and table latencies.
-// 16 warps of 128 registers hide those better than 12 of 152 with the j weights double
+// 346 -> 151 us; the shared-memory pipe is 82 % busy (ncu, 2,000 x 1,000), the rest are branch and
+// table latencies.  16 warps of 128 registers hide those better than 12 of 152 with the j weights double
 // buffered (7.4 ms).  Small matrices run a few warps per CTA, so that their tiles reach all SMs.
 constexpr int SB = 10, SJ = 32, SCH = 64, SSTG = 2, SWARPS_MAX = 16;
 constexpr int SROW = SJ * SB;  // floats of a sample's j weights
